@@ -26,6 +26,7 @@
 namespace rq {
 
 constexpr int kStackTotal = 64;  // entries per lane (shared + local)
+constexpr int kDeeperMinLanes = 16;  // any-hit: lanes that make a second node step worth its issue slots
 
 #ifdef RQ_MAXNREG
 #define RQ_KERNEL_BOUNDS __maxnreg__(RQ_MAXNREG)  // register cap (occupancy experiments)
@@ -327,12 +328,19 @@ __global__ void RQ_KERNEL_BOUNDS cwbvh_kernel(const TraceParams p) {
                 }
                 if (fault) finish(fault);
             }
-            // Any-hit: a lane whose node produced no triangles and has inner
-            // children left descends once more in the same iteration, in the
-            // order the next iteration would take (+2 % batched any-hit;
-            // closest-hit loses 6-10 %: its triangle tests, which shrink
-            // tmax, get postponed more often).
-            if (ANY && __ballot_sync(kFullMask, active && tg.y == 0u && ng.y > 0x00FFFFFFu)) {
+            // Any-hit: lanes whose node produced no triangles and has inner
+            // children left descend once more in the same iteration, in the
+            // order the next iteration would take, when at least half of the
+            // warp would: the second node test costs the warp its full ~285
+            // instructions however few lanes take it.  12 scenes / 20M AO
+            // rays 3,570 us with it taken for any lane, 3,565 / 3,552 / 3,525
+            // / 3,484 / 3,510 / 3,588 us from 4 / 8 / 12 / 16 / 20 / 24 lanes
+            // on; 10,592 triangles / 1M rays 220.7 -> 217 us, 8M triangles /
+            // 16M rays 5,050 -> 4,976 us.  Taken again while as many lanes
+            // would: no gain over once.  Closest-hit loses 1-3 % with any of
+            // these limits (its triangle tests, which shrink tmax, get
+            // postponed more often).
+            if (ANY && __popc(__ballot_sync(kFullMask, active && tg.y == 0u && ng.y > 0x00FFFFFFu)) >= kDeeperMinLanes) {
                 if (active && tg.y == 0u && ng.y > 0x00FFFFFFu) {
                     const unsigned f2 = node_step();
                     if (f2) finish(f2);
