@@ -17,6 +17,7 @@ struct rq_batch {
     rq_query query = RQ_ANY;
     rq_bvh_kind kind = RQ_BVH_CWBVH;
     rq_launch launch{};
+    bool free_shape = false;  // no launch shape was asked for
     rq_batch_params params{};
     std::vector<rq::TraceItem> items;  // host copy (ray_begin = global prefix)
     rq::TraceItem* d_items = nullptr;
@@ -34,14 +35,12 @@ static rq_status batch_enqueue(rq_batch* b, cudaStream_t s) {
         rq_status st = sort_plan_run(b->plan, s);
         if (st != RQ_OK) return st;
     }
-    rq_status st = reset_counter(b->ctx, s);
-    if (st != RQ_OK) return st;
     TraceParams p = base_params(b->ctx, b->launch);
     p.single = b->items.empty() ? TraceItem{} : b->items[0];
     p.items = b->d_items;
     p.n_items = (int)b->items.size();
     p.total_rays = b->total;
-    return launch_trace(b->kind, b->query, b->launch, true, false, p, s);
+    return launch_trace(b->kind, b->query, b->launch, true, false, b->free_shape, p, s);
 }
 
 }  // namespace rq
@@ -68,6 +67,7 @@ rq_status rq_batch_create(rq_ctx_t ctx, const rq_batch_item* items, int n_items,
     if (params) b->params = *params;
     else b->params.sort_threshold = -1;
     b->launch = resolve_launch(kind, query, params ? &params->launch : nullptr);
+    b->free_shape = launch_unset(params ? &params->launch : nullptr);
 
     std::vector<TraceItem> to_sort;
     std::vector<float> bounds;
@@ -140,14 +140,12 @@ rq_status rq_batch_run_stage(rq_batch_t b, int stage, void* stream) {
     if (!b || stage < 1 || stage > 2) return RQ_ERR_INVALID_ARG;
     cudaStream_t s = (cudaStream_t)stream;
     if (stage == 1) return b->sorted_any ? sort_plan_run(b->plan, s) : RQ_OK;
-    rq_status st = reset_counter(b->ctx, s);
-    if (st != RQ_OK) return st;
     TraceParams p = base_params(b->ctx, b->launch);
     p.single = b->items.empty() ? TraceItem{} : b->items[0];
     p.items = b->d_items;
     p.n_items = (int)b->items.size();
     p.total_rays = b->total;
-    return launch_trace(b->kind, b->query, b->launch, true, false, p, s);
+    return launch_trace(b->kind, b->query, b->launch, true, false, b->free_shape, p, s);
 }
 
 int rq_batch_kernel_count(rq_batch_t b) {

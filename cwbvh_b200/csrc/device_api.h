@@ -77,6 +77,10 @@ typedef void (*TraceKernelFn)(TraceParams);
 constexpr int64_t kRingMinRaysPerThread = 64;
 constexpr int64_t kRingMinRaysPerThreadSingle = 256;
 TraceKernelFn trace_kernel(rq_bvh_kind kind, bool any, int smem, bool multi, bool count, bool ring);
+// The CWBVH kernel with g = 8 or 4 lanes to a ray for small launches (see
+// trace.cu), launched with lanes_block() threads per lanes_block() / g rays.
+TraceKernelFn lanes_kernel(bool any, bool multi, int g);
+int lanes_block();
 int smem_entries_of(int requested);
 size_t trace_smem_bytes(rq_bvh_kind kind, int smem_entries, int block, bool ring);
 

@@ -84,11 +84,39 @@ static int blocks_per_sm(TraceKernelFn fn, int block, size_t smem) {
     return cache[key];
 }
 
-rq_status launch_trace(rq_bvh_kind kind, rq_query q, const rq_launch& l, bool multi, bool count,
+bool launch_unset(const rq_launch* l) {
+    return !l || (l->block_size == 0 && l->blocks_per_sm == 0 && l->smem_stack == 0 && l->postpone_ratio == 0.f &&
+                  l->fetch_nd == 0 && l->fetch_nw == 0);
+}
+
+// Lanes that share a ray in a CWBVH launch of `rays` rays (0: a lane per ray,
+// the persistent kernel).  Whole calls on 10,592 triangles, us, with
+// 8 lanes / 4 lanes / one, 148 SMs: closest-hit 4,096 rays 24.8 / 29.2 / 50.5,
+// 16,384 30.7 / 33.8 / 53.8, 32,768 49.4 / 39.4 / 55.7, 65,536 85.6 / 69.0 /
+// 62.2; any-hit bakes 4,096 30.5 / 32.8 / 53.4, 16,384 35.8 / 37.9 / 61.1,
+// 65,536 67.6 / 59.5 / 66.9, 262,144 230 / 183 / 128.  (Two lanes to a ray are
+// never the fastest.)
+static int lanes_per_ray(rq_query q, int64_t rays, int sms) {
+    if (rays <= 128 * (int64_t)sms) return 8;
+    return rays <= (q == RQ_ANY ? 448 : 320) * (int64_t)sms ? 4 : 0;
+}
+
+rq_status launch_trace(rq_bvh_kind kind, rq_query q, const rq_launch& l, bool multi, bool count, bool free_shape,
                        const TraceParams& p, cudaStream_t s) {
     if (p.total_rays <= 0) return RQ_OK;
+    void* args[] = {(void*)&p};
     int dev = 0;
     RQ_CUDA(cudaGetDevice(&dev));
+    if (free_shape && kind == RQ_BVH_CWBVH && !count) {
+        if (const int g = lanes_per_ray(q, p.total_rays, device_sms(dev))) {
+            const int64_t rays_per_block = lanes_block() / g;
+            const unsigned blocks = (unsigned)((p.total_rays + rays_per_block - 1) / rays_per_block);
+            RQ_CUDA(cudaLaunchKernel((const void*)lanes_kernel(q == RQ_ANY, multi, g), dim3(blocks),
+                                     dim3((unsigned)lanes_block()), args, 0, s));
+            return RQ_OK;
+        }
+    }
+    RQ_CUDA(cudaMemsetAsync(&p.scratch->ray_counter, 0, sizeof(unsigned long long), s));
     // Any-hit launches with many rays per thread take the ring-prefetching kernel.
     TraceKernelFn fn = nullptr;
     size_t smem = 0;
@@ -109,7 +137,6 @@ rq_status launch_trace(rq_bvh_kind kind, rq_query q, const rq_launch& l, bool mu
     const int64_t warps_needed = (p.total_rays + 31) / 32;
     const int64_t blocks_needed = (warps_needed * 32 + l.block_size - 1) / l.block_size;
     grid = std::max<int64_t>(1, std::min(grid, blocks_needed));
-    void* args[] = {(void*)&p};
     RQ_CUDA(cudaLaunchKernel((const void*)fn, dim3((unsigned)grid), dim3((unsigned)l.block_size), args, smem, s));
     return RQ_OK;
 }
@@ -365,10 +392,7 @@ static rq_status trace_impl(rq_ctx_t ctx, rq_scene_t scene, const rq_ray* rays, 
     p.single.ao_counts = ao_counts;
     p.single.ao_spp = ao_spp;
     if (speculative >= 0) p.bvh2_speculative = speculative;
-    cudaStream_t s = (cudaStream_t)stream;
-    rq_status st = reset_counter(ctx, s);
-    if (st != RQ_OK) return st;
-    return launch_trace(scene->kind, query, l, false, nv != nullptr, p, s);
+    return launch_trace(scene->kind, query, l, false, nv != nullptr, launch_unset(launch), p, (cudaStream_t)stream);
 }
 
 rq_status rq_trace(rq_ctx_t ctx, rq_scene_t scene, const rq_ray* rays, rq_hit* hits, int64_t count, rq_query query,

@@ -256,14 +256,13 @@ void rq_server::launch_batch(Worker& w, std::vector<Piece*>& batch, int32_t batc
     if (st == RQ_OK)
         ok(cudaMemcpyAsync(w.d_items, w.h_items, batch.size() * sizeof(rq::TraceItem), cudaMemcpyHostToDevice,
                            w.stream));
-    if (st == RQ_OK) st = rq::reset_counter(w.ctx, w.stream);
     if (st == RQ_OK) {
         rq::TraceParams p = rq::base_params(w.ctx, launch);
         p.single = w.h_items[0];
         p.items = w.d_items;
         p.n_items = (int)batch.size();
         p.total_rays = ray_begin;
-        st = rq::launch_trace(kind, params.query, launch, true, false, p, w.stream);
+        st = rq::launch_trace(kind, params.query, launch, true, false, rq::launch_unset(&params.launch), p, w.stream);
     }
     for (Piece* pc : batch) {
         Req* r = pc->req;

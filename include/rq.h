@@ -58,7 +58,10 @@ typedef enum rq_bvh_kind { RQ_BVH_CWBVH = 0, RQ_BVH_BVH2 = 1 } rq_bvh_kind;
 typedef enum rq_query { RQ_CLOSEST = 0, RQ_ANY = 1 } rq_query;
 
 /* Launch parameters of the persistent trace kernels.  Zero fields take the
- * built-in defaults (or the autotuner's cached choice, see rq_autotune). */
+ * built-in defaults (or the autotuner's cached choice, see rq_autotune).  With
+ * none of the shape, postponing and fetch fields set, a CWBVH launch of a few
+ * ten thousand rays or fewer takes a kernel with several lanes per ray
+ * instead; step_limit holds for it too. */
 typedef struct rq_launch {
     int block_size;       /* threads per block: 64, 128, 256 or 512             */
     int blocks_per_sm;    /* persistent grid = SMs x this (0 = occupancy max)   */
