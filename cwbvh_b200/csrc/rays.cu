@@ -43,53 +43,110 @@ __device__ inline float3 cross3(float3 a, float3 b) {
 __device__ inline float len3(float3 a) { return sqrtf(a.x * a.x + a.y * a.y + a.z * a.z); }
 __device__ inline float3 norm3(float3 a) { return mul3(a, 1.0f / len3(a)); }
 
+// A whole ray as one 32-byte store (st.v8, sm_100): two 16-byte stores fill
+// their sectors by halves and cost the L2 two writes per sector.  `wide`: the
+// buffer is 32-byte aligned (the interface asks for 16).
+__device__ __forceinline__ void store_ray(Ray* r, float4 o, float4 d, bool wide) {
+    if (wide) {
+        asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(r), "f"(o.x), "f"(o.y), "f"(o.z),
+                     "f"(o.w), "f"(d.x), "f"(d.y), "f"(d.z), "f"(d.w)
+                     : "memory");
+    } else {
+        r->origin_tmin = o;
+        r->dir_tmax = d;
+    }
+}
+static bool aligned32(const void* p) { return ((uintptr_t)p & 31u) == 0; }
+
+// Division of 31-bit numbers by one divisor: floor(i / d) = i * mul >> shift
+// with mul = ceil(2^shift / d) and shift = 31 + ceil(log2 d) is exact for every
+// i < 2^31 (Granlund and Montgomery, "Division by Invariant Integers using
+// Multiplication", PLDI 1994), mul < 2^32.
+struct FastDiv {
+    uint32_t mul, shift, d;
+    explicit FastDiv(uint32_t divisor) : d(divisor) {
+        uint32_t l = 0;
+        while (l < 31 && (1ull << l) < divisor) ++l;
+        shift = 31 + l;
+        mul = (uint32_t)(((1ull << shift) + divisor - 1) / divisor);
+    }
+    __device__ uint32_t div(uint32_t i) const { return (uint32_t)((uint64_t)i * mul >> shift); }
+};
+
+// Surfel frame in shared memory: normal, tangents, ray origin.
+struct SurfelFrame {
+    float3 n, t1, t2, o;
+};
+
+constexpr int kAoBlock = 256;
+
 // One ray per (surfel, sample), surfel = i / spp: tangent frame from n x z
 // (n x y when that is short), concentric disk lifted to the cosine
 // hemisphere, origin pushed off the surface by radius * offset_scale
 // (src/ValidationKernels.cu:41-101).  The random stream of ray i is keyed by
 // its index first_ray + i in the whole request, so a request generated in
 // pieces gives the same rays as in one call.
-__global__ void aorays_kernel(const float4* __restrict__ pos, const float4* __restrict__ nrm,
-                              const float* __restrict__ radius, int64_t n_rays, int spp, int64_t first_ray,
-                              uint32_t k0, uint32_t k1, float tmin, float tmax, float offset_scale,
-                              Ray* __restrict__ out) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n_rays) return;
-    const int64_t s = i / spp;
-    const float3 p = f3(pos[s]);
-    const float3 n = f3(nrm[s]);
-    const float r = radius ? radius[s] : 0.0f;
+//
+// Bound by instruction issue (277 warp instructions for 32 rays of 32 B), so
+// what a surfel's rays share is computed once: the block's first threads make
+// its surfels' frames in shared memory, and the ray threads read them.  A
+// block's rays start `skip` samples into its first surfel.  16M rays at 4 per
+// surfel 199 -> 159 us, 1M at 32 per surfel 16.6 -> 12.7 us, the same bits.
+template <bool SMALL>
+__global__ void __launch_bounds__(kAoBlock) aorays_kernel(
+        const float4* __restrict__ pos, const float4* __restrict__ nrm, const float* __restrict__ radius,
+        int64_t n_rays, FastDiv spp, int64_t first_ray, uint32_t k0, uint32_t k1, float tmin, float tmax,
+        float offset_scale, Ray* __restrict__ out, bool wide) {
+    __shared__ SurfelFrame frames[kAoBlock];
+    const int64_t block0 = (int64_t)blockIdx.x * kAoBlock;
+    const int64_t surfel0 = SMALL ? (int64_t)spp.div((uint32_t)block0) : block0 / spp.d;  // SMALL: n_rays < 2^31
+    const uint32_t skip = (uint32_t)(block0 - surfel0 * spp.d);
+    const uint32_t here = (uint32_t)(n_rays - block0 < kAoBlock ? n_rays - block0 : kAoBlock);  // rays of the block
+    // skip + here - 1 < spp + 256 <= 2^31: spp fits an int
+    const uint32_t n_surfels = spp.div(skip + here - 1u) + 1u;
+    if (threadIdx.x < n_surfels) {
+        const int64_t s = surfel0 + threadIdx.x;
+        const float3 p = f3(pos[s]);
+        const float3 n = f3(nrm[s]);
+        const float r = radius ? radius[s] : 0.0f;
+        float3 t1 = cross3(n, make_float3(0.f, 0.f, 1.f));
+        if (len3(t1) < 0.1f) t1 = cross3(n, make_float3(0.f, 1.f, 0.f));
+        t1 = norm3(t1);
+        const float3 t2 = norm3(cross3(t1, n));
+        SurfelFrame& f = frames[threadIdx.x];
+        f.n = n;
+        f.t1 = t1;
+        f.t2 = t2;
+        const bool none = n.x == 0.f && n.y == 0.f && n.z == 0.f;
+        f.o = none ? p : add3(p, mul3(n, r * offset_scale));
+    }
+    __syncthreads();
+    if (threadIdx.x >= here) return;
+    const int64_t i = block0 + threadIdx.x;
+    const SurfelFrame& f = frames[spp.div(skip + threadIdx.x)];
+    const float3 n = f.n, o = f.o;
     if (n.x == 0.f && n.y == 0.f && n.z == 0.f) {  // no surface (a primary miss): an empty ray
-        out[i].origin_tmin = make_float4(p.x, p.y, p.z, 0.f);
-        out[i].dir_tmax = make_float4(0.f, 0.f, 1.f, 0.f);
+        store_ray(out + i, make_float4(o.x, o.y, o.z, 0.f), make_float4(0.f, 0.f, 1.f, 0.f), wide);
         return;
     }
-    float3 t1 = cross3(n, make_float3(0.f, 0.f, 1.f));
-    if (len3(t1) < 0.1f) t1 = cross3(n, make_float3(0.f, 1.f, 0.f));
-    t1 = norm3(t1);
-    const float3 t2 = norm3(cross3(t1, n));
     const uint64_t ctr = (uint64_t)(first_ray + i);
     const U4 rnd = philox4x32_10(U4{(uint32_t)ctr, (uint32_t)(ctr >> 32), 0u, 0u}, k0, k1);
     const float a = 2.0f * unit24(rnd.x) - 1.0f, b = 2.0f * unit24(rnd.y) - 1.0f;
     float dxl = 0.f, dyl = 0.f;
     if (a != 0.f || b != 0.f) {
         const float kPi = 3.1415926f;
-        float rr, th;
-        if (a * a > b * b) {
-            rr = a;
-            th = (kPi / 4.0f) * (b / a);
-        } else {
-            rr = b;
-            th = (kPi / 2.0f) - (kPi / 4.0f) * (a / b);
-        }
-        dxl = rr * cosf(th);
-        dyl = rr * sinf(th);
+        const bool x_major = a * a > b * b;
+        const float rr = x_major ? a : b;
+        const float q = (x_major ? b : a) / rr;
+        const float th = x_major ? __fmul_rn(kPi / 4.0f, q) : __fmaf_rn(-(kPi / 4.0f), q, kPi / 2.0f);
+        float sn, cs;
+        sincosf(th, &sn, &cs);
+        dxl = rr * cs;
+        dyl = rr * sn;
     }
     const float dzl = sqrtf(fmaxf(0.0f, 1.0f - dxl * dxl - dyl * dyl));
-    const float3 d = norm3(add3(add3(mul3(t1, dxl), mul3(t2, dyl)), mul3(n, dzl)));
-    const float3 o = add3(p, mul3(n, r * offset_scale));
-    out[i].origin_tmin = make_float4(o.x, o.y, o.z, tmin);
-    out[i].dir_tmax = make_float4(d.x, d.y, d.z, tmax);
+    const float3 d = norm3(add3(add3(mul3(f.t1, dxl), mul3(f.t2, dyl)), mul3(n, dzl)));
+    store_ray(out + i, make_float4(o.x, o.y, o.z, tmin), make_float4(d.x, d.y, d.z, tmax), wide);
 }
 
 // Surfel i on triangle floor(u * nt) at barycentrics (1 - sqrt(a), b sqrt(a)).
@@ -118,21 +175,39 @@ __global__ void surfels_kernel(const float* __restrict__ v, const int32_t* __res
 // Ray i is pixel (x, y) of tile i / (tw * th), tiles row-major across the
 // image and pixels row-major within a tile (tw = width, th = 1: the image
 // row-major).
+//
+// Bound by the 32 B written per ray: 4.2M rays 36.6 -> 21.3 us (6.3 TB/s) with
+// whole-sector stores.  The four divisions that place a pixel are
+// multiplications (FastDiv); images of 2^31 pixels and more divide.
+template <bool SMALL>
 __global__ void camera_rays_kernel(float3 eye, float3 fwd, float3 right, float3 upv, float half_w, float half_h,
-                                   int width, int height, int tw, int th, float tmin, float tmax,
-                                   Ray* __restrict__ out) {
+                                   int width, int height, int tw, int th, FastDiv per_tile, FastDiv tiles_x,
+                                   FastDiv tile_w, float tmin, float tmax, Ray* __restrict__ out,
+                                   bool wide) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (int64_t)width * height) return;
-    const int64_t tile = i / ((int64_t)tw * th);
-    const int in_tile = (int)(i % ((int64_t)tw * th));
-    const int tiles_x = width / tw;
-    const int x = (int)(tile % tiles_x) * tw + in_tile % tw;
-    const int y = (int)(tile / tiles_x) * th + in_tile / tw;
+    int tile_x, tile_y, in_x, in_y;
+    if (SMALL) {
+        const uint32_t tile = per_tile.div((uint32_t)i), in_tile = (uint32_t)i - tile * per_tile.d;
+        const uint32_t ty = tiles_x.div(tile), iy = tile_w.div(in_tile);
+        tile_x = (int)(tile - ty * tiles_x.d);
+        tile_y = (int)ty;
+        in_x = (int)(in_tile - iy * tile_w.d);
+        in_y = (int)iy;
+    } else {
+        const int64_t tile = i / ((int64_t)tw * th), in_tile = i - tile * ((int64_t)tw * th);
+        const int across = width / tw;
+        tile_x = (int)(tile % across);
+        tile_y = (int)(tile / across);
+        in_x = (int)(in_tile % tw);
+        in_y = (int)(in_tile / tw);
+    }
+    const int x = tile_x * tw + in_x;
+    const int y = tile_y * th + in_y;
     const float sx = ((x + 0.5f) / width * 2.0f - 1.0f) * half_w;
     const float sy = (1.0f - (y + 0.5f) / height * 2.0f) * half_h;
     const float3 d = norm3(add3(add3(fwd, mul3(right, sx)), mul3(upv, sy)));
-    out[i].origin_tmin = make_float4(eye.x, eye.y, eye.z, tmin);
-    out[i].dir_tmax = make_float4(d.x, d.y, d.z, tmax);
+    store_ray(out + i, make_float4(eye.x, eye.y, eye.z, tmin), make_float4(d.x, d.y, d.z, tmax), wide);
 }
 
 // Hit point and facing geometric normal of each closest hit.
@@ -158,13 +233,22 @@ __global__ void surfels_from_hits_kernel(const Ray* __restrict__ rays, const Hit
     if (radius) radius[i] = 0.0f;
 }
 
-// Fraction of a surfel's spp rays whose hit id is not -1.
+// Fraction of a surfel's spp rays whose hit id is not -1.  A memory-bound sum:
+// P lanes (the largest power of two that leaves each four hits, at most 32)
+// take a surfel's hits side by side, four loads in flight each, and add up:
+// 16M hits at 32 per surfel 63.8 -> 39.2 us (6.5 TB/s of the hits' sectors),
+// 128 surfels 4.1 -> 2 us; a thread per surfel below 8 rays as before.
+template <int P>
 __global__ void ao_reduce_kernel(const Hit* __restrict__ hits, int64_t n_surfels, int spp, float* __restrict__ ao) {
-    const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= n_surfels) return;
+    const int64_t s = (int64_t)blockIdx.x * (blockDim.x / P) + threadIdx.x / P;
+    const int c = (int)(threadIdx.x % P);
     int occ = 0;
-    for (int k = 0; k < spp; ++k) occ += __float_as_int(hits[s * spp + k].t_triId_u_v.y) != -1;
-    ao[s] = (float)occ / (float)spp;
+    if (s < n_surfels)
+#pragma unroll 4
+        for (int k = c; k < spp; k += P) occ += __float_as_int(hits[s * spp + k].t_triId_u_v.y) != -1;
+#pragma unroll
+    for (int m = P / 2; m > 0; m >>= 1) occ += __shfl_xor_sync(kFullMask, occ, m);
+    if (c == 0 && s < n_surfels) ao[s] = (float)occ / (float)spp;
 }
 
 // ----------------------------------------------------------------- sorting
@@ -229,9 +313,10 @@ rq_status aorays_launch(const float* pos, const float* nrm, const float* radius,
         return RQ_ERR_INVALID_ARG;
     const int64_t n = n_surfels * spp;
     if (n == 0) return RQ_OK;
-    aorays_kernel<<<blocks_for(n, 256), 256, 0, (cudaStream_t)stream>>>(
-        (const float4*)pos, (const float4*)nrm, radius, n, spp, first_ray, (uint32_t)seed, (uint32_t)(seed >> 32),
-        tmin, tmax, offset_scale, (Ray*)out_rays);
+    const auto kernel = n < ((int64_t)1 << 31) ? aorays_kernel<true> : aorays_kernel<false>;
+    kernel<<<blocks_for(n, kAoBlock), kAoBlock, 0, (cudaStream_t)stream>>>(
+        (const float4*)pos, (const float4*)nrm, radius, n, FastDiv((uint32_t)spp), first_ray, (uint32_t)seed, (uint32_t)(seed >> 32),
+        tmin, tmax, offset_scale, (Ray*)out_rays, aligned32(out_rays));
     RQ_CUDA(cudaGetLastError());
     return RQ_OK;
 }
@@ -363,9 +448,12 @@ static rq_status camera_rays_impl(const float eye[3], const float look[3], const
     const float half_h = std::tan(vfov_deg * 0.5f * 3.14159265358979f / 180.0f);
     const float half_w = half_h * (float)width / (float)height;
     const int64_t n = (int64_t)width * height;
-    camera_rays_kernel<<<blocks_for(n, 256), 256, 0, (cudaStream_t)stream>>>(e, fwd, right, upv, half_w, half_h, width,
-                                                                             height, tw, th, tmin, tmax,
-                                                                             (Ray*)out_rays);
+    const bool small = n < ((int64_t)1 << 31);
+    const FastDiv per_tile(small ? (uint32_t)(tw * th) : 1u), tiles_x((uint32_t)(width / tw)), tile_w((uint32_t)tw);
+    const auto kernel = small ? camera_rays_kernel<true> : camera_rays_kernel<false>;
+    kernel<<<blocks_for(n, 256), 256, 0, (cudaStream_t)stream>>>(e, fwd, right, upv, half_w, half_h, width, height,
+                                                                 tw, th, per_tile, tiles_x, tile_w, tmin, tmax,
+                                                                 (Ray*)out_rays, aligned32(out_rays));
     RQ_CUDA(cudaGetLastError());
     return RQ_OK;
 }
@@ -395,8 +483,13 @@ rq_status rq_surfels_from_hits(rq_scene_t scene, const rq_ray* rays, const rq_hi
 rq_status rq_ao_reduce(const rq_hit* hits, int64_t n_surfels, int spp, float* out_ao, void* stream) {
     if (n_surfels < 0 || spp <= 0 || (n_surfels > 0 && (!hits || !out_ao))) return RQ_ERR_INVALID_ARG;
     if (n_surfels == 0) return RQ_OK;
-    ao_reduce_kernel<<<blocks_for(n_surfels, 256), 256, 0, (cudaStream_t)stream>>>((const Hit*)hits, n_surfels, spp,
-                                                                                   out_ao);
+    int lanes = 1;
+    while (lanes < 32 && 8 * lanes <= spp) lanes *= 2;
+    const auto kernel = lanes == 32 ? ao_reduce_kernel<32> : lanes == 16 ? ao_reduce_kernel<16>
+                      : lanes == 8 ? ao_reduce_kernel<8> : lanes == 4 ? ao_reduce_kernel<4>
+                      : lanes == 2 ? ao_reduce_kernel<2> : ao_reduce_kernel<1>;
+    kernel<<<blocks_for(n_surfels * lanes, 256), 256, 0, (cudaStream_t)stream>>>((const Hit*)hits, n_surfels, spp,
+                                                                                 out_ao);
     RQ_CUDA(cudaGetLastError());
     return RQ_OK;
 }
