@@ -262,23 +262,10 @@ __device__ inline uint32_t spread10(uint32_t x) {
     return x;
 }
 
-// 32-bit ray key: 3 x 9-bit Morton code of the origin inside the item's
-// bounds (high 27 bits) then the direction octant (low 3 bits); the item
-// number sits above it so every item's rays stay together.
-__global__ void morton_keys_kernel(const TraceItem* __restrict__ items, int n_items, const float* __restrict__ bounds,
-                                   int64_t total, uint64_t* __restrict__ keys, int32_t* __restrict__ vals) {
-    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= total) return;
-    int lo = 0, hi = n_items - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (items[mid].ray_begin <= g) lo = mid; else hi = mid - 1;
-    }
-    const TraceItem& it = items[lo];
-    const int64_t k = g - it.ray_begin;
-    const float4 o = it.rays[k].origin_tmin;
-    const float4 d = it.rays[k].dir_tmax;
-    const float* b = bounds + 6 * lo;
+// 30-bit ray key: 3 x 9-bit Morton code of the origin inside the bounds
+// b (high 27 bits) then the direction octant (low 3 bits).
+constexpr int kRayKeyBits = 30;
+__device__ inline uint32_t ray_key(const float4& o, const float4& d, const float* b) {
     uint32_t q[3];
     const float oo[3] = {o.x, o.y, o.z};
 #pragma unroll
@@ -290,7 +277,23 @@ __global__ void morton_keys_kernel(const TraceItem* __restrict__ items, int n_it
     }
     const uint32_t m = (spread10(q[0]) << 2) | (spread10(q[1]) << 1) | spread10(q[2]);
     const uint32_t oct = (d.x < 0.f ? 4u : 0u) | (d.y < 0.f ? 2u : 0u) | (d.z < 0.f ? 1u : 0u);
-    keys[g] = ((uint64_t)lo << 32) | ((uint64_t)m << 3) | oct;
+    return (m << 3) | oct;
+}
+
+// Keys of the rays of several items: the item number sits above the ray key,
+// so every item's rays stay together.
+__global__ void morton_keys_kernel(const TraceItem* __restrict__ items, int n_items, const float* __restrict__ bounds,
+                                   int64_t total, uint64_t* __restrict__ keys, int32_t* __restrict__ vals) {
+    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= total) return;
+    int lo = 0, hi = n_items - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (items[mid].ray_begin <= g) lo = mid; else hi = mid - 1;
+    }
+    const TraceItem& it = items[lo];
+    const int64_t k = g - it.ray_begin;
+    keys[g] = ((uint64_t)lo << 32) | ray_key(it.rays[k].origin_tmin, it.rays[k].dir_tmax, bounds + 6 * lo);
     vals[g] = (int32_t)k;
 }
 
@@ -302,6 +305,53 @@ __global__ void gather_rays_kernel(const TraceItem* __restrict__ items, const ui
     const Ray* src = items[item].rays + vals[g];
     sorted[g].origin_tmin = __ldg(&src->origin_tmin);
     sorted[g].dir_tmax = __ldg(&src->dir_tmax);
+}
+
+// The same for one ray buffer: 32-bit keys (four radix passes of 8-byte pairs
+// instead of five of 12), bounds in the launch arguments, and rays moved as
+// one 32-byte load and store each (`wide`: both buffers 32-byte aligned).
+// Both kernels are bound by their bytes; the gather reads its rays in Morton
+// order, a sector at a time, and keeps four of them in flight per thread.
+struct Bounds6 {
+    float b[6];
+};
+
+__device__ __forceinline__ void load_ray(const Ray* r, float4& o, float4& d, bool wide) {
+    if (wide) {
+        asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+            : "=f"(o.x), "=f"(o.y), "=f"(o.z), "=f"(o.w), "=f"(d.x), "=f"(d.y), "=f"(d.z), "=f"(d.w)
+            : "l"(r));
+    } else {
+        o = __ldg(&r->origin_tmin);
+        d = __ldg(&r->dir_tmax);
+    }
+}
+
+__global__ void ray_keys_kernel(const Ray* __restrict__ rays, Bounds6 bounds, int64_t n, uint32_t* __restrict__ keys,
+                                int32_t* __restrict__ vals, bool wide) {
+    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= n) return;
+    float4 o, d;
+    load_ray(rays + g, o, d, wide);
+    keys[g] = ray_key(o, d, bounds.b);
+    vals[g] = (int32_t)g;
+}
+
+constexpr int kGatherRays = 4;
+__global__ void permute_rays_kernel(const Ray* __restrict__ rays, const int32_t* __restrict__ perm, int64_t n,
+                                    Ray* __restrict__ sorted, bool wide_in, bool wide_out) {
+    const int64_t base = (int64_t)blockIdx.x * (blockDim.x * kGatherRays) + threadIdx.x;
+    float4 o[kGatherRays], d[kGatherRays];
+#pragma unroll
+    for (int q = 0; q < kGatherRays; ++q) {
+        const int64_t g = base + (int64_t)q * blockDim.x;
+        if (g < n) load_ray(rays + perm[g], o[q], d[q], wide_in);
+    }
+#pragma unroll
+    for (int q = 0; q < kGatherRays; ++q) {
+        const int64_t g = base + (int64_t)q * blockDim.x;
+        if (g < n) store_ray(sorted + g, o[q], d[q], wide_out);
+    }
 }
 
 static unsigned blocks_for(int64_t n, int b) { return (unsigned)((n + b - 1) / b); }
@@ -494,27 +544,78 @@ rq_status rq_ao_reduce(const rq_hit* hits, int64_t n_surfels, int spp, float* ou
     return RQ_OK;
 }
 
+// The buffers of a sort are kept with the context between calls up to
+// kSortKeepBytes (about 20M rays; allocating them, and counting a plan's
+// kernels, cost ten times the sort), and given back with it; a larger sort
+// allocates its own.  The call ends with its stream synchronized, so the next
+// one finds them free; calls on one context from several threads take turns.
+constexpr size_t kSortKeepBytes = (size_t)256 << 20;
+
 rq_status rq_sort_rays(rq_ctx_t ctx, const rq_ray* rays, int64_t count, const float bounds_lo[3],
                        const float bounds_hi[3], rq_ray* sorted_rays, int32_t* perm, void* stream) {
     if (!ctx || count < 0 || (count > 0 && (!rays || !sorted_rays || !perm || !bounds_lo || !bounds_hi)))
         return RQ_ERR_INVALID_ARG;
     if (count == 0) return RQ_OK;
     cudaStream_t s = (cudaStream_t)stream;
-    TraceItem it{};
-    it.rays = (const Ray*)rays;
-    it.count = count;
-    SortPlan plan;
-    std::vector<float> b = {bounds_lo[0], bounds_lo[1], bounds_lo[2], bounds_hi[0], bounds_hi[1], bounds_hi[2]};
-    rq_status st = sort_plan_create({it}, b, plan);
-    if (st == RQ_OK) st = sort_plan_run(plan, s);
-    if (st == RQ_OK) {
-        cudaError_t e = cudaMemcpyAsync(sorted_rays, plan.sorted, (size_t)count * sizeof(Ray), cudaMemcpyDeviceToDevice, s);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(perm, plan.vals_out, (size_t)count * 4, cudaMemcpyDeviceToDevice, s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) st = cuda_fail(e, "rq_sort_rays");
+    const size_t n = (size_t)count;
+    // Outputs that overlap the input or each other are written last, from copies.
+    auto overlap = [](const void* a, size_t an, const void* b, size_t bn) {
+        return (uintptr_t)a < (uintptr_t)b + bn && (uintptr_t)b < (uintptr_t)a + an;
+    };
+    const bool staged = overlap(rays, n * sizeof(Ray), sorted_rays, n * sizeof(Ray)) ||
+                        overlap(rays, n * sizeof(Ray), perm, n * 4) ||
+                        overlap(sorted_rays, n * sizeof(Ray), perm, n * 4);
+    size_t cub_bytes = 0;
+    RQ_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, cub_bytes, (const uint32_t*)nullptr, (uint32_t*)nullptr,
+                                            (const int32_t*)nullptr, (int32_t*)nullptr, count, 0, kRayKeyBits, s));
+    size_t bytes = 0;
+    auto take = [&](size_t b) {
+        const size_t at = bytes;
+        bytes += (b + 255) / 256 * 256;
+        return at;
+    };
+    const size_t keys_in = take(n * 4), keys_out = take(n * 4), vals_in = take(n * 4), cub_temp = take(cub_bytes);
+    const size_t st_rays = staged ? take(n * sizeof(Ray)) : 0, st_perm = staged ? take(n * 4) : 0;
+
+    std::lock_guard<std::mutex> lk(ctx->temp_mu);
+    int dev = 0;
+    RQ_CUDA(cudaGetDevice(&dev));
+    char* base = nullptr;
+    const bool keep = bytes <= kSortKeepBytes && dev == ctx->device;
+    if (keep) {
+        if (ctx->temp_bytes < bytes) {
+            cudaFree(ctx->temp);
+            ctx->temp = nullptr;
+            ctx->temp_bytes = 0;
+            RQ_CUDA(cudaMalloc(&ctx->temp, bytes));
+            ctx->temp_bytes = bytes;
+        }
+        base = (char*)ctx->temp;
+    } else {
+        RQ_CUDA(cudaMalloc(&base, bytes));
     }
-    sort_plan_destroy(plan);
-    return st;
+    int32_t* const out_perm = staged ? (int32_t*)(base + st_perm) : perm;
+    Ray* const out_rays = staged ? (Ray*)(base + st_rays) : (Ray*)sorted_rays;
+    const Bounds6 b{{bounds_lo[0], bounds_lo[1], bounds_lo[2], bounds_hi[0], bounds_hi[1], bounds_hi[2]}};
+    ray_keys_kernel<<<blocks_for(count, 256), 256, 0, s>>>((const Ray*)rays, b, count, (uint32_t*)(base + keys_in),
+                                                           (int32_t*)(base + vals_in), aligned32(rays));
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess)
+        e = cub::DeviceRadixSort::SortPairs(base + cub_temp, cub_bytes, (const uint32_t*)(base + keys_in),
+                                            (uint32_t*)(base + keys_out), (const int32_t*)(base + vals_in), out_perm,
+                                            count, 0, kRayKeyBits, s);
+    if (e == cudaSuccess) {
+        permute_rays_kernel<<<blocks_for(count, 256 * kGatherRays), 256, 0, s>>>(
+            (const Ray*)rays, out_perm, count, out_rays, aligned32(rays), aligned32(out_rays));
+        e = cudaGetLastError();
+    }
+    if (staged && e == cudaSuccess)
+        e = cudaMemcpyAsync(sorted_rays, out_rays, n * sizeof(Ray), cudaMemcpyDeviceToDevice, s);
+    if (staged && e == cudaSuccess) e = cudaMemcpyAsync(perm, out_perm, n * 4, cudaMemcpyDeviceToDevice, s);
+    const cudaError_t done = cudaStreamSynchronize(s);  // also after an error: the buffers are reused or freed
+    if (e == cudaSuccess) e = done;
+    if (!keep) cudaFree(base);
+    return e == cudaSuccess ? RQ_OK : cuda_fail(e, "rq_sort_rays");
 }
 
 }  // extern "C"

@@ -12,8 +12,9 @@
 struct rq_ctx {
     int device = 0;
     rq::DevScratch* scratch = nullptr;  // device
-    void* temp = nullptr;               // grow-on-demand device temp (sorting)
+    void* temp = nullptr;               // sort buffers kept between rq_sort_rays calls
     size_t temp_bytes = 0;
+    std::mutex temp_mu;                 // held by a call that uses them
 };
 
 struct rq_scene {

@@ -303,7 +303,10 @@ rq_status rq_ao_reduce(const rq_hit* hits, int64_t n_surfels, int spp, float* ou
 /* ---------------------------------------------------------- Morton sorting */
 /* Sort rays by a 32-bit key (10-bit Morton per origin axis inside the given
  * bounds, high bits; direction octant, low bits).  Writes the sorted rays and
- * the permutation (sorted position -> original index). */
+ * the permutation (sorted position -> original index); waits for the stream.
+ * Sort buffers of up to 256 MB (about 20M rays) stay with the context until
+ * it is destroyed; larger ones are allocated and freed by the call.  Outputs
+ * may overlap the input or each other. */
 rq_status rq_sort_rays(rq_ctx_t ctx, const rq_ray* rays, int64_t count, const float bounds_lo[3],
                        const float bounds_hi[3], rq_ray* sorted_rays, int32_t* perm,
                        void* stream);
@@ -312,7 +315,7 @@ rq_status rq_sort_rays(rq_ctx_t ctx, const rq_ray* rays, int64_t count, const fl
  * reference.  Some callers cannot call cudaMalloc -- a plugin inside a host
  * that owns all device memory through its own pool, a service whose
  * device-memory budget was fixed at start-up -- and rq_sort_rays allocates
- * its sort buffers on every call.  This entry point keeps its scratch in one
+ * its sort buffers when they grow.  This entry point keeps its scratch in one
  * static 20 MiB device array that every GPU loading librq holds until exit,
  * which limits a call to RQ_SORT_STATIC_MAX_RAYS rays (larger counts return
  * RQ_ERR_INVALID_ARG with the limit in rq_last_error).  Outputs are identical
