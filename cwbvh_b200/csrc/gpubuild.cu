@@ -35,19 +35,30 @@
 #include <cfloat>
 #include <cmath>
 #include <cstring>
+#include <utility>
+#include <vector>
 
 #include "runtime.h"
 
 namespace rq {
 namespace {
 
-struct BNode {
+// A box with the SAH cost and the triangle count of what it bounds: two
+// 16-byte loads give all that a walk up the tree reads of a child.
+struct __align__(16) NodeBox {
+    float lo[3];
+    float cost;  // SAH cost of the subtree
+    float hi[3];
+    int32_t count;  // triangles below
+};
+
+struct __align__(16) BNode {
     int32_t left, right;  // >= 0: internal node, < 0: leaf ~(sorted position)
     int32_t parent;       // -1 at the root
-    int32_t count;        // triangles below
-    float lo[3], hi[3];
-    float cost;           // SAH cost of the subtree
+    int32_t pad;
+    NodeBox b;
 };
+static_assert(sizeof(NodeBox) == 32 && sizeof(BNode) == 48, "node layout");
 
 // SAH weights of the treelet restructuring (Karras and Aila 2013).
 constexpr float kCt = 1.2f;  // per node
@@ -427,25 +438,50 @@ __device__ inline float node_cost(float area, float c0, float c1) {
     return __fadd_rn(__fadd_rn(__fmul_rn(kCt, area), c0), c1);
 }
 
-__device__ inline void child_box(const BNode* nodes, const uint64_t* k, uint64_t idx_mask, const float* v,
-                                 const int32_t* idx, int32_t code, float lo[3], float hi[3], int32_t& count,
-                                 float* cost = nullptr) {
-    if (code >= 0) {
-        const volatile BNode& c = nodes[code];
-        for (int a = 0; a < 3; ++a) { lo[a] = c.lo[a]; hi[a] = c.hi[a]; }
-        count = c.count;
-        if (cost) *cost = c.cost;
-    } else {
-        tri_box(v, idx, key_tri(k, ~code, idx_mask), lo, hi);
-        count = 1;
-        if (cost) *cost = __fmul_rn(kCi, half_area(lo, hi));
+// The box of a child: a node's, or that of the leaf at a sorted position.
+// Boxes other threads of the same launch may have written are read from L2
+// (ld.cg), never from a possibly stale L1 line.
+__device__ inline NodeBox child_box(const BNode* nodes, const NodeBox* leaves, int32_t code) {
+    const float4* p = reinterpret_cast<const float4*>(code >= 0 ? &nodes[code].b : &leaves[~code]);
+    const float4 x = __ldcg(p), y = __ldcg(p + 1);
+    NodeBox b;
+    b.lo[0] = x.x; b.lo[1] = x.y; b.lo[2] = x.z; b.cost = x.w;
+    b.hi[0] = y.x; b.hi[1] = y.y; b.hi[2] = y.z; b.count = __float_as_int(y.w);
+    return b;
+}
+__device__ inline void store_box(NodeBox* to, const NodeBox& b) {
+    float4* p = reinterpret_cast<float4*>(to);
+    p[0] = make_float4(b.lo[0], b.lo[1], b.lo[2], b.cost);
+    p[1] = make_float4(b.hi[0], b.hi[1], b.hi[2], __int_as_float(b.count));
+}
+// The box of a node over two children, its count and its cost.
+__device__ inline NodeBox join(const NodeBox& l, const NodeBox& r) {
+    NodeBox b;
+    for (int a = 0; a < 3; ++a) {
+        b.lo[a] = fminf(l.lo[a], r.lo[a]);
+        b.hi[a] = fmaxf(l.hi[a], r.hi[a]);
     }
+    b.count = l.count + r.count;
+    b.cost = node_cost(half_area(b.lo, b.hi), l.cost, r.cost);
+    return b;
+}
+
+// The boxes of the leaves in sorted order.
+__global__ void leaf_boxes_kernel(const uint64_t* k, uint64_t idx_mask, int64_t n, const float* v, const int32_t* idx,
+                                  NodeBox* leaves) {
+    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= n) return;
+    NodeBox b;
+    tri_box(v, idx, key_tri(k, p, idx_mask), b.lo, b.hi);
+    b.cost = __fmul_rn(kCi, half_area(b.lo, b.hi));
+    b.count = 1;
+    store_box(leaves + p, b);
 }
 
 // Boxes and counts bottom-up: the second of a node's two children to arrive
 // completes it and goes on to the parent.
-__global__ void boxes_kernel(const uint64_t* k, uint64_t idx_mask, int64_t n, const float* v, const int32_t* idx,
-                             BNode* nodes, const int32_t* leaf_parent, int32_t* arrivals) {
+__global__ void boxes_kernel(int64_t n, const NodeBox* leaves, BNode* nodes, const int32_t* leaf_parent,
+                             int32_t* arrivals) {
     const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n) return;
     int32_t node = leaf_parent[p];
@@ -453,20 +489,8 @@ __global__ void boxes_kernel(const uint64_t* k, uint64_t idx_mask, int64_t n, co
         __threadfence();
         if (atomicAdd(&arrivals[node], 1) == 0) return;  // the sibling finishes this node
         __threadfence();
-        float l0[3], h0[3], l1[3], h1[3], k0, k1;
-        int32_t c0, c1;
-        child_box(nodes, k, idx_mask, v, idx, nodes[node].left, l0, h0, c0, &k0);
-        child_box(nodes, k, idx_mask, v, idx, nodes[node].right, l1, h1, c1, &k1);
-        volatile BNode& nd = nodes[node];
-        float lo[3], hi[3];
-        for (int a = 0; a < 3; ++a) {
-            lo[a] = fminf(l0[a], l1[a]);
-            hi[a] = fmaxf(h0[a], h1[a]);
-            nd.lo[a] = lo[a];
-            nd.hi[a] = hi[a];
-        }
-        nd.count = c0 + c1;
-        nd.cost = node_cost(half_area(lo, hi), k0, k1);
+        store_box(&nodes[node].b, join(child_box(nodes, leaves, nodes[node].left),
+                                       child_box(nodes, leaves, nodes[node].right)));
         node = nodes[node].parent;
     }
 }
@@ -481,14 +505,12 @@ __global__ void boxes_kernel(const uint64_t* k, uint64_t idx_mask, int64_t n, co
 // is processed only when both its children are final.
 constexpr int kTreeletLeaves = 7;
 
-// Node fields other threads of the same launch may have rewritten are read
-// from L2 (ld.cg), never from a possibly stale L1 line.
+// Links other threads of the same launch may have rewritten are read from L2.
 __device__ inline int32_t ld_left(const BNode* nodes, int32_t x) { return __ldcg(&nodes[x].left); }
 __device__ inline int32_t ld_right(const BNode* nodes, int32_t x) { return __ldcg(&nodes[x].right); }
 __device__ inline int32_t ld_parent(const BNode* nodes, int32_t x) { return __ldcg(&nodes[x].parent); }
 
-__device__ void restructure(BNode* nodes, const uint64_t* k, uint64_t idx_mask, const float* v, const int32_t* idx,
-                            int32_t* leaf_parent, int32_t root) {
+__device__ void restructure(BNode* nodes, const NodeBox* leaves, int32_t* leaf_parent, int32_t root) {
     int32_t inner[kTreeletLeaves - 1], leaf[kTreeletLeaves];
     float larea[kTreeletLeaves];
     int n_in = 1, n_leaf = 2;
@@ -497,10 +519,16 @@ __device__ void restructure(BNode* nodes, const uint64_t* k, uint64_t idx_mask, 
     leaf[1] = ld_right(nodes, root);
     float llo[kTreeletLeaves][3], lhi[kTreeletLeaves][3], lcost[kTreeletLeaves];
     int32_t lcnt[kTreeletLeaves];
-    for (int q = 0; q < 2; ++q) {
-        child_box(nodes, k, idx_mask, v, idx, leaf[q], llo[q], lhi[q], lcnt[q], &lcost[q]);
-        larea[q] = half_area(llo[q], lhi[q]);
-    }
+    auto take = [&](int q, int32_t code) {
+        const NodeBox b = child_box(nodes, leaves, code);
+        leaf[q] = code;
+        for (int a = 0; a < 3; ++a) { llo[q][a] = b.lo[a]; lhi[q][a] = b.hi[a]; }
+        lcost[q] = b.cost;
+        lcnt[q] = b.count;
+        larea[q] = half_area(b.lo, b.hi);
+    };
+    take(0, leaf[0]);
+    take(1, leaf[1]);
     while (n_leaf < kTreeletLeaves) {
         int best = -1;
         float ba = -1.f;
@@ -510,12 +538,8 @@ __device__ void restructure(BNode* nodes, const uint64_t* k, uint64_t idx_mask, 
         const int32_t x = leaf[best];
         inner[n_in++] = x;
         const int32_t l = ld_left(nodes, x), r = ld_right(nodes, x);
-        leaf[best] = l;
-        child_box(nodes, k, idx_mask, v, idx, l, llo[best], lhi[best], lcnt[best], &lcost[best]);
-        larea[best] = half_area(llo[best], lhi[best]);
-        leaf[n_leaf] = r;
-        child_box(nodes, k, idx_mask, v, idx, r, llo[n_leaf], lhi[n_leaf], lcnt[n_leaf], &lcost[n_leaf]);
-        larea[n_leaf] = half_area(llo[n_leaf], lhi[n_leaf]);
+        take(best, l);
+        take(n_leaf, r);
         ++n_leaf;
     }
     if (n_leaf < 3) return;
@@ -552,7 +576,7 @@ __device__ void restructure(BNode* nodes, const uint64_t* k, uint64_t idx_mask, 
         cost[S] = __fadd_rn(__fmul_rn(kCt, half_area(slo, shi)), best);
         part[S] = (uint8_t)bp;
     }
-    if (!(cost[full] < 0.999f * __ldcg(&nodes[root].cost))) return;
+    if (!(cost[full] < 0.999f * __ldcg(&nodes[root].b.cost))) return;
     // every subset the new tree splits must have a split (finite costs); check
     // before writing anything
     {
@@ -596,19 +620,18 @@ __device__ void restructure(BNode* nodes, const uint64_t* k, uint64_t idx_mask, 
         BNode& b = nodes[nd];
         b.left = code[0];
         b.right = code[1];
-        float slo[3], shi[3];
-        subset_box(S, slo, shi);
-        for (int a = 0; a < 3; ++a) { b.lo[a] = slo[a]; b.hi[a] = shi[a]; }
-        int32_t cnt = 0;
+        NodeBox nb;
+        subset_box(S, nb.lo, nb.hi);
+        nb.count = 0;
         for (int q = 0; q < n_leaf; ++q)
-            if (S & (1 << q)) cnt += lcnt[q];
-        b.count = cnt;
-        b.cost = cost[S];
+            if (S & (1 << q)) nb.count += lcnt[q];
+        nb.cost = cost[S];
+        store_box(&b.b, nb);
     }
 }
 
-__global__ void treelet_kernel(const uint64_t* k, uint64_t idx_mask, int64_t n, const float* v, const int32_t* idx,
-                               BNode* nodes, int32_t* leaf_parent, int32_t* arrivals, int min_count) {
+__global__ void treelet_kernel(int64_t n, const NodeBox* leaves, BNode* nodes, int32_t* leaf_parent, int32_t* arrivals,
+                               int min_count) {
     const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n) return;
     int32_t node = leaf_parent[p];
@@ -617,15 +640,10 @@ __global__ void treelet_kernel(const uint64_t* k, uint64_t idx_mask, int64_t n, 
         if (atomicAdd(&arrivals[node], 1) == 0) return;
         __threadfence();
         // this node's cost from its (final) children, then its treelet
-        float l0[3], h0[3], l1[3], h1[3], k0, k1;
-        int32_t c0, c1;
-        child_box(nodes, k, idx_mask, v, idx, ld_left(nodes, node), l0, h0, c0, &k0);
-        child_box(nodes, k, idx_mask, v, idx, ld_right(nodes, node), l1, h1, c1, &k1);
-        volatile BNode& nd = nodes[node];
-        float lo[3], hi[3];
-        for (int a = 0; a < 3; ++a) { lo[a] = fminf(l0[a], l1[a]); hi[a] = fmaxf(h0[a], h1[a]); }
-        nd.cost = node_cost(half_area(lo, hi), k0, k1);
-        if (c0 + c1 >= min_count) restructure(nodes, k, idx_mask, v, idx, leaf_parent, node);
+        const NodeBox b = join(child_box(nodes, leaves, ld_left(nodes, node)),
+                               child_box(nodes, leaves, ld_right(nodes, node)));
+        __stcg(&nodes[node].b.cost, b.cost);
+        if (b.count >= min_count) restructure(nodes, leaves, leaf_parent, node);
         node = ld_parent(nodes, node);
     }
 }
@@ -665,7 +683,7 @@ constexpr SubsetTable make_subset_table() {
 __constant__ SubsetTable c_subsets = make_subset_table();
 
 struct TreeletSmem {
-    float llo[kTreeletLeaves][3], lhi[kTreeletLeaves][3], lcost[kTreeletLeaves];
+    float llo[kTreeletLeaves][3], lhi[kTreeletLeaves][3];
     int32_t lcnt[kTreeletLeaves], leaf[kTreeletLeaves], inner[kTreeletLeaves - 1];
     float cost[1 << kTreeletLeaves];
     float slo[1 << kTreeletLeaves][3], shi[1 << kTreeletLeaves][3];  // subset boxes
@@ -704,19 +722,18 @@ __device__ void subset_box_s(TreeletSmem& t, int S, float lo[3], float hi[3]) {
 }
 
 // The whole warp restructures the treelet rooted at `root` (warp-uniform).
-__device__ void restructure_warp(BNode* nodes, const uint64_t* k, uint64_t idx_mask, const float* v,
-                                 const int32_t* idx, int32_t* leaf_parent, int32_t root, float root_cost,
-                                 TreeletSmem& t) {
+__device__ void restructure_warp(BNode* nodes, const NodeBox* leaves, int32_t* leaf_parent, int32_t root,
+                                 float root_cost, TreeletSmem& t) {
     const unsigned lane = threadIdx.x & 31u;
     // Grow the treelet: lane q holds leaf q.
     int32_t my_leaf = -1;
-    float mlo[3] = {0.f, 0.f, 0.f}, mhi[3] = {0.f, 0.f, 0.f}, mcost = 0.f, marea = -1.f;
-    int32_t mcnt = 0;
+    NodeBox mine{};
+    float marea = -1.f;
     int n_in = 1, n_leaf = 2;
     if (lane < 2) {
         my_leaf = lane == 0 ? ld_left(nodes, root) : ld_right(nodes, root);
-        child_box(nodes, k, idx_mask, v, idx, my_leaf, mlo, mhi, mcnt, &mcost);
-        marea = half_area(mlo, mhi);
+        mine = child_box(nodes, leaves, my_leaf);
+        marea = half_area(mine.lo, mine.hi);
     }
     if (lane == 0) t.inner[0] = root;
     while (n_leaf < kTreeletLeaves) {
@@ -734,23 +751,22 @@ __device__ void restructure_warp(BNode* nodes, const uint64_t* k, uint64_t idx_m
         ++n_in;
         if ((int)lane == best || (int)lane == n_leaf) {
             my_leaf = (int)lane == best ? ld_left(nodes, x) : ld_right(nodes, x);
-            child_box(nodes, k, idx_mask, v, idx, my_leaf, mlo, mhi, mcnt, &mcost);
-            marea = half_area(mlo, mhi);
+            mine = child_box(nodes, leaves, my_leaf);
+            marea = half_area(mine.lo, mine.hi);
         }
         ++n_leaf;
     }
     if (n_leaf < 3) return;
     if ((int)lane < n_leaf) {
         for (int a = 0; a < 3; ++a) {
-            t.llo[lane][a] = mlo[a];
-            t.lhi[lane][a] = mhi[a];
-            t.slo[1 << lane][a] = mlo[a];
-            t.shi[1 << lane][a] = mhi[a];
+            t.llo[lane][a] = mine.lo[a];
+            t.lhi[lane][a] = mine.hi[a];
+            t.slo[1 << lane][a] = mine.lo[a];
+            t.shi[1 << lane][a] = mine.hi[a];
         }
-        t.lcost[lane] = mcost;
-        t.lcnt[lane] = mcnt;
+        t.lcnt[lane] = mine.count;
         t.leaf[lane] = my_leaf;
-        t.cost[1 << lane] = mcost;
+        t.cost[1 << lane] = mine.cost;
         t.part[1 << lane] = 0;
     }
     __syncwarp();
@@ -850,12 +866,13 @@ __device__ void restructure_warp(BNode* nodes, const uint64_t* k, uint64_t idx_m
                 BNode& b = nodes[nd];
                 b.left = code[0];
                 b.right = code[1];
-                for (int a = 0; a < 3; ++a) { b.lo[a] = t.slo[S][a]; b.hi[a] = t.shi[S][a]; }
-                int32_t cnt = 0;
+                NodeBox nb;
+                for (int a = 0; a < 3; ++a) { nb.lo[a] = t.slo[S][a]; nb.hi[a] = t.shi[S][a]; }
+                nb.count = 0;
                 for (int q = 0; q < n_leaf; ++q)
-                    if (S & (1 << q)) cnt += t.lcnt[q];
-                b.count = cnt;
-                b.cost = t.cost[S];
+                    if (S & (1 << q)) nb.count += t.lcnt[q];
+                nb.cost = t.cost[S];
+                store_box(&b.b, nb);
             }
             __threadfence();
         }
@@ -866,8 +883,7 @@ __device__ void restructure_warp(BNode* nodes, const uint64_t* k, uint64_t idx_m
 constexpr int kTreeletWarpBlock = 128;
 
 __global__ void __launch_bounds__(kTreeletWarpBlock) treelet_warp_kernel(
-        const uint64_t* k, uint64_t idx_mask, int64_t n, const float* v, const int32_t* idx, BNode* nodes,
-        int32_t* leaf_parent, int32_t* arrivals, int min_count) {
+        int64_t n, const NodeBox* leaves, BNode* nodes, int32_t* leaf_parent, int32_t* arrivals, int min_count) {
     __shared__ TreeletSmem smem[kTreeletWarpBlock / 32];
     TreeletSmem& t = smem[threadIdx.x / 32];
     const unsigned lane = threadIdx.x & 31u;
@@ -884,16 +900,11 @@ __global__ void __launch_bounds__(kTreeletWarpBlock) treelet_warp_kernel(
         float cost = 0.f;
         bool due = false;
         if (go) {
-            float l0[3], h0[3], l1[3], h1[3], k0, k1;
-            int32_t c0, c1;
-            child_box(nodes, k, idx_mask, v, idx, ld_left(nodes, node), l0, h0, c0, &k0);
-            child_box(nodes, k, idx_mask, v, idx, ld_right(nodes, node), l1, h1, c1, &k1);
-            volatile BNode& nd = nodes[node];
-            float lo[3], hi[3];
-            for (int a = 0; a < 3; ++a) { lo[a] = fminf(l0[a], l1[a]); hi[a] = fmaxf(h0[a], h1[a]); }
-            cost = node_cost(half_area(lo, hi), k0, k1);
-            nd.cost = cost;
-            due = c0 + c1 >= min_count;
+            const NodeBox b = join(child_box(nodes, leaves, ld_left(nodes, node)),
+                                   child_box(nodes, leaves, ld_right(nodes, node)));
+            cost = b.cost;
+            __stcg(&nodes[node].b.cost, cost);
+            due = b.count >= min_count;
         }
         unsigned want = __ballot_sync(kWarpAll, due);
         while (want) {
@@ -901,7 +912,7 @@ __global__ void __launch_bounds__(kTreeletWarpBlock) treelet_warp_kernel(
             want &= want - 1;
             const int32_t root = __shfl_sync(kWarpAll, node, src);
             const float rc = __shfl_sync(kWarpAll, cost, src);
-            restructure_warp(nodes, k, idx_mask, v, idx, leaf_parent, root, rc, t);
+            restructure_warp(nodes, leaves, leaf_parent, root, rc, t);
         }
         if (go) node = ld_parent(nodes, node);
         if (__ballot_sync(kWarpAll, node >= 0) == 0u) break;
@@ -954,10 +965,14 @@ struct Item {
     int32_t addr;  // 8-wide node index
 };
 
-struct Ctr {
-    unsigned long long nodes;  // 8-wide nodes allocated
-    unsigned long long tris;   // triangle slots allocated
-    unsigned long long next;   // items of the next level
+// Counters of the expansion.  alloc[L]: 8-wide nodes of level L in the low
+// word, triangle slots taken by level L - 1 in the high word (one atomic takes
+// both); node_base[L] / tri_base[L]: nodes / triangle slots of the levels before.
+constexpr int kMaxLevels = 4096;
+struct Levels {
+    unsigned long long alloc[kMaxLevels + 1];
+    unsigned int node_base[kMaxLevels + 1];
+    unsigned int tri_base[kMaxLevels + 1];
     unsigned int error;
 };
 
@@ -972,15 +987,14 @@ struct Ctr {
 constexpr float kCollapseNode = 1.0f;  // per 8-wide node, times its area
 constexpr float kCollapseLeaf = 0.3f;  // per triangle in a leaf, times the leaf's area
 
-struct CollapseDP {
+struct __align__(16) CollapseDP {
     float best[8];    // k = 1..8
     uint8_t how[8];   // 0 leaf, 1 own node, 2 + j opened with j slots to the left child
     uint8_t split8;   // slots to the left child when the node is an 8-wide node of its own
     uint8_t pad[7];
 };
 
-__global__ void collapse_dp_kernel(const uint64_t* k, uint64_t idx_mask, int64_t n, const float* v,
-                                   const int32_t* idx, const BNode* nodes, const int32_t* leaf_parent,
+__global__ void collapse_dp_kernel(int64_t n, const NodeBox* leaves, const BNode* nodes, const int32_t* leaf_parent,
                                    int32_t* arrivals, CollapseDP* dp) {
     const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n) return;
@@ -990,22 +1004,22 @@ __global__ void collapse_dp_kernel(const uint64_t* k, uint64_t idx_mask, int64_t
         if (atomicAdd(&arrivals[node], 1) == 0) return;  // the sibling finishes this node
         __threadfence();
         const int32_t c[2] = {__ldcg(&nodes[node].left), __ldcg(&nodes[node].right)};
-        float cost[2][9], area[2];
-        int32_t cnt[2];
+        float cost[2][9];
+        int32_t prims = 0;
         for (int q = 0; q < 2; ++q) {
-            float lo[3], hi[3];
-            child_box(nodes, k, idx_mask, v, idx, c[q], lo, hi, cnt[q]);
-            area[q] = half_area(lo, hi);
-            for (int kk = 1; kk <= 8; ++kk)
-                cost[q][kk] = c[q] >= 0 ? __ldcg(&dp[c[q]].best[kk - 1]) : kCollapseLeaf * area[q];
+            const NodeBox b = child_box(nodes, leaves, c[q]);
+            prims += b.count;
+            if (c[q] >= 0) {
+                const float4* best = reinterpret_cast<const float4*>(dp[c[q]].best);
+                const float4 x = __ldcg(best), y = __ldcg(best + 1);
+                cost[q][1] = x.x; cost[q][2] = x.y; cost[q][3] = x.z; cost[q][4] = x.w;
+                cost[q][5] = y.x; cost[q][6] = y.y; cost[q][7] = y.z; cost[q][8] = y.w;
+            } else {
+                for (int kk = 1; kk <= 8; ++kk) cost[q][kk] = kCollapseLeaf * half_area(b.lo, b.hi);
+            }
         }
-        float lo[3], hi[3];
-        for (int a = 0; a < 3; ++a) {
-            lo[a] = __ldcg(&nodes[node].lo[a]);
-            hi[a] = __ldcg(&nodes[node].hi[a]);
-        }
-        const float av = half_area(lo, hi);
-        const int32_t prims = cnt[0] + cnt[1];
+        const NodeBox own = child_box(nodes, leaves, node);
+        const float av = half_area(own.lo, own.hi);
         float open[9];
         uint8_t split[9];
         for (int kk = 2; kk <= 8; ++kk) {
@@ -1032,177 +1046,259 @@ __global__ void collapse_dp_kernel(const uint64_t* k, uint64_t idx_mask, int64_t
     }
 }
 
-// Expands the binary nodes of one level into 8-wide nodes, their slots as
-// the collapse chose them.
-__global__ void expand_kernel(const Item* items, int64_t n_items, Item* next, int64_t next_cap, const BNode* nodes,
-                              const uint64_t* k, uint64_t idx_mask, const float* v, const int32_t* idx,
-                              const float* tv, const int32_t* tidx, const int32_t* ref_tri, float4* out_nodes,
-                              int64_t node_cap, float4* woop, int32_t* prim, int64_t tri_cap, Ctr* ctr,
-                              const CollapseDP* dp) {
-    const int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (w >= n_items) return;
-    const Item it = items[w];
-    int32_t code[8];
-    float clo[8][3], chi[8][3];
-    int32_t cnt[8];
-    int m = 0;
-    if (it.code < 0) {  // one triangle: the root holds one leaf
-        code[0] = it.code;
-        child_box(nodes, k, idx_mask, v, idx, it.code, clo[0], chi[0], cnt[0]);
-        m = 1;
-    } else if (dp) {
-        // the slots the collapse chose: (binary child, slots it fills), left first
-        int32_t stc[16];
-        int stk[16];
-        int sp = 0;
-        const BNode& b = nodes[it.code];
-        const int s8 = dp[it.code].split8;
-        stc[sp] = b.right; stk[sp++] = 8 - s8;
-        stc[sp] = b.left; stk[sp++] = s8;
-        while (sp > 0) {
-            --sp;
-            const int32_t x = stc[sp];
-            const int kk = stk[sp];
-            const int h = (x >= 0 && kk >= 1 && kk <= 8) ? dp[x].how[kk - 1] : 0;
-            if (h >= 2) {
-                const int j = h - 2;
-                if (sp + 2 > 16 || j < 1 || j >= kk) {  // a table the recursion cannot follow
-                    atomicOr(&ctr->error, 4u);
-                    return;
-                }
-                stc[sp] = nodes[x].right; stk[sp++] = kk - j;
-                stc[sp] = nodes[x].left; stk[sp++] = j;
+// Expands the binary nodes of one level into 8-wide nodes, their slots as the
+// collapse chose them.  Eight lanes to a node, one per child: a thread per
+// node spent 200-400 us on a level of any size, a chain of a few thousand
+// dependent loads and steps with 6 of 32 lanes at work.  A binary node that
+// fills k slots owns k neighbouring lanes; opening it hands its right part to
+// the lane where that part begins, so children come out in depth-first order
+// without a stack, and sums, votes and minima run over the eight lanes.  The
+// level's item count is read on the device, so the host queues levels ahead.
+// 10 levels of a 500,000-triangle heightfield: 2,204 -> 155 us
+// (with eight levels queued past the last).
+constexpr int kExpandBlock = 128;
+
+__global__ void __launch_bounds__(kExpandBlock) expand_kernel(
+        int level, const Item* items, Item* next, const BNode* nodes, const NodeBox* leaves, const uint64_t* k,
+        uint64_t idx_mask, const int32_t* ref_tri, float4* out_nodes, unsigned node_cap, int32_t* prim,
+        unsigned tri_cap, Levels* lv, const CollapseDP* dp) {
+    constexpr int kGroups = kExpandBlock / 8;
+    __shared__ float4 node_smem[kGroups][5];
+    __shared__ int32_t open_code[kGroups][8];
+    __shared__ int open_slots[kGroups][8];
+    const unsigned lane = threadIdx.x & 31u, shift = lane & 24u;
+    const int c = (int)(lane & 7u), group = (int)(threadIdx.x >> 3);
+    // Levels queued behind one that failed have nothing valid to read.
+    if (lv->error) return;
+    // Where this level's triangles and the next one's nodes begin: after all
+    // that the levels before took.
+    const unsigned n_items = (unsigned)lv->alloc[level];
+    const unsigned next0 = lv->node_base[level] + n_items;
+    const unsigned tri0 = level ? lv->tri_base[level - 1] + (unsigned)(lv->alloc[level] >> 32) : 0u;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        lv->node_base[level + 1] = next0;
+        lv->tri_base[level] = tri0;
+    }
+    auto octet = [&](bool b) -> unsigned { return (__ballot_sync(kWarpAll, b) >> shift) & 0xFFu; };
+    auto all_or = [&](unsigned x) -> unsigned {
+        for (int m = 4; m > 0; m >>= 1) x |= __shfl_xor_sync(kWarpAll, x, m);
+        return x;
+    };
+    const unsigned groups = gridDim.x * kGroups;
+    // warp-uniform loop: the groups of a warp take neighbouring items
+    for (unsigned w0 = blockIdx.x * kGroups + (threadIdx.x >> 5) * 4; w0 < n_items; w0 += groups) {
+        const unsigned w = w0 + (shift >> 3);
+        const bool active = w < n_items;
+        unsigned err = 0u;
+        Item it{0, 0};
+        if (active) it = items[w];
+        // ---- the children: lane q holds the binary node whose slots begin at q
+        bool has = false;
+        int32_t code = 0;
+        int slots = 0;
+        if (active) {
+            if (it.code < 0) {  // one triangle: the root holds one leaf
+                has = c == 0;
+                code = it.code;
+                slots = 8;
             } else {
-                if (m >= 8) {
-                    atomicOr(&ctr->error, 4u);
-                    return;
+                const int s8 = dp[it.code].split8;
+                const int2 lr = *reinterpret_cast<const int2*>(&nodes[it.code].left);
+                if (s8 < 1 || s8 > 7) {
+                    err = 4u;
+                } else if (c == 0) {
+                    has = true;
+                    code = lr.x;
+                    slots = s8;
+                } else if (c == s8) {
+                    has = true;
+                    code = lr.y;
+                    slots = 8 - s8;
                 }
-                code[m] = x;
-                child_box(nodes, k, idx_mask, v, idx, x, clo[m], chi[m], cnt[m]);
-                ++m;
             }
         }
-    } else {
-        atomicOr(&ctr->error, 4u);  // an inner node needs the collapse table
-        return;
-    }
-    // node box
-    float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-    for (int c = 0; c < m; ++c)
-        for (int a = 0; a < 3; ++a) { lo[a] = fminf(lo[a], clo[c][a]); hi[a] = fmaxf(hi[a], chi[c][a]); }
-    // octant slots: cheapest (slot, child) pairs first, as the host converter
-    float nc[3];
-    for (int a = 0; a < 3; ++a) nc[a] = (lo[a] + hi[a]) * 0.5f;
-    int slot_of[8], child_in[8];
-    bool slot_free[8];
-    for (int s = 0; s < 8; ++s) { slot_of[s] = -1; slot_free[s] = true; child_in[s] = -1; }
-    for (;;) {
-        float best = FLT_MAX;
-        int bs = -1, bc = -1;
-        for (int s = 0; s < 8; ++s) {
-            if (!slot_free[s]) continue;
-            const float dx = (s & 4) ? -1.f : 1.f, dy = (s & 2) ? -1.f : 1.f, dz = (s & 1) ? -1.f : 1.f;
-            for (int c = 0; c < m; ++c) {
-                if (slot_of[c] >= 0) continue;
-                const float cx = __fsub_rn(__fmul_rn(__fadd_rn(clo[c][0], chi[c][0]), 0.5f), nc[0]);
-                const float cy = __fsub_rn(__fmul_rn(__fadd_rn(clo[c][1], chi[c][1]), 0.5f), nc[1]);
-                const float cz = __fsub_rn(__fmul_rn(__fadd_rn(clo[c][2], chi[c][2]), 0.5f), nc[2]);
-                const float cost = __fadd_rn(__fadd_rn(__fmul_rn(cx, dx), __fmul_rn(cy, dy)), __fmul_rn(cz, dz));
-                if (cost < best) { best = cost; bs = s; bc = c; }
+        for (int step = 0; step < 8; ++step) {
+            const int how = has && code >= 0 && slots >= 1 ? dp[code].how[slots - 1] : 0;
+            bool open = how >= 2;
+            const int j = how - 2;
+            if (open && (j < 1 || j >= slots || step == 7)) {  // a table that opens more than it has slots
+                err = 4u;
+                open = false;
             }
+            if (!__any_sync(kWarpAll, open)) break;
+            open_slots[group][c] = 0;
+            __syncwarp();
+            if (open) {
+                const int2 lr = *reinterpret_cast<const int2*>(&nodes[code].left);
+                open_code[group][c + j] = lr.y;
+                open_slots[group][c + j] = slots - j;
+                code = lr.x;
+                slots = j;
+            }
+            __syncwarp();
+            if (open_slots[group][c]) {
+                has = true;
+                code = open_code[group][c];
+                slots = open_slots[group][c];
+            }
+            __syncwarp();
         }
-        if (bs < 0) break;
-        slot_free[bs] = false;
-        slot_of[bc] = bs;
-        child_in[bs] = bc;
-    }
-    // per-axis exponent, grown while a child's upper bound does not fit a byte
-    int e[3];
-    for (int a = 0; a < 3; ++a) {
-        const float r = ceilf(log2f((hi[a] - lo[a]) / 255.0f));
-        e[a] = isfinite(r) ? (int)fmaxf(-127.f, fminf(127.f, r)) : 0;
-        for (;;) {
-            const float scale = ldexpf(1.0f, e[a]);
-            bool fits = true;
-            for (int c = 0; c < m; ++c)
-                if ((int)ceilf((chi[c][a] - lo[a]) / scale) > 255) fits = false;
-            if (fits || e[a] >= 127) break;
-            ++e[a];
-        }
-    }
-    // allocations: inner children as one block, leaf triangles as one run
-    int n_inner = 0, n_tris = 0;
-    for (int c = 0; c < m; ++c) {
-        if (cnt[c] > 3) ++n_inner;
-        else n_tris += cnt[c];
-    }
-    const unsigned long long base = n_inner ? atomicAdd(&ctr->nodes, (unsigned long long)n_inner) : 0ull;
-    const unsigned long long tbase = n_tris ? atomicAdd(&ctr->tris, (unsigned long long)n_tris) : 0ull;
-    const unsigned long long qbase = n_inner ? atomicAdd(&ctr->next, (unsigned long long)n_inner) : 0ull;
-    if (base + n_inner > (unsigned long long)node_cap || tbase + n_tris > (unsigned long long)tri_cap ||
-        qbase + n_inner > (unsigned long long)next_cap) {
-        atomicOr(&ctr->error, 1u);
-        return;
-    }
-    float4 node[5];
-    for (int q = 0; q < 5; ++q) node[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-    unsigned char* bytes = reinterpret_cast<unsigned char*>(node);
-    uint8_t imask = 0;
-    int inner = 0, leaf_tris = 0;
-    for (int s = 0; s < 8; ++s) {
-        const int c = child_in[s];
-        if (c < 0) continue;
+        NodeBox b{};
+        if (has) b = child_box(nodes, leaves, code);
+        // ---- node box
+        float lo[3], hi[3];
         for (int a = 0; a < 3; ++a) {
-            const float scale = ldexpf(1.0f, e[a]);
-            bytes[32 + s + 8 * a] = (uint8_t)(int)floorf((clo[c][a] - lo[a]) / scale);
-            bytes[32 + s + 8 * (3 + a)] = (uint8_t)(int)ceilf((chi[c][a] - lo[a]) / scale);
+            lo[a] = has ? b.lo[a] : FLT_MAX;
+            hi[a] = has ? b.hi[a] : -FLT_MAX;
+            for (int m = 4; m > 0; m >>= 1) {
+                lo[a] = fminf(lo[a], __shfl_xor_sync(kWarpAll, lo[a], m));
+                hi[a] = fmaxf(hi[a], __shfl_xor_sync(kWarpAll, hi[a], m));
+            }
         }
-        if (cnt[c] > 3) {
-            imask |= (uint8_t)(1u << s);
-            bytes[24 + s] = (uint8_t)((1u << 5) | (24u + s));
-            next[qbase + inner] = Item{code[c], (int32_t)(base + inner)};
-            ++inner;
-        } else {
-            const uint32_t unary = cnt[c] == 1 ? 1u : (cnt[c] == 2 ? 3u : 7u);
-            bytes[24 + s] = (uint8_t)((unary << 5) | ((uint32_t)leaf_tris & 31u));
-            // the child's triangles: a leaf, or a subtree of at most 3
-            int32_t st[4];
-            int sp = 0;
-            st[sp++] = code[c];
-            while (sp > 0) {
-                const int32_t x = st[--sp];
-                if (leaf_tris >= n_tris || (x >= 0 && sp + 2 > 4)) {  // counts disagree with the tree
-                    atomicOr(&ctr->error, 2u);
-                    return;
+        // ---- octant slots: cheapest (slot, child) pairs first, as the host
+        // converter; equal costs to the lower slot, then the lower child
+        float nc[3], cc[3];
+        for (int a = 0; a < 3; ++a) {
+            nc[a] = (lo[a] + hi[a]) * 0.5f;
+            cc[a] = __fsub_rn(__fmul_rn(__fadd_rn(b.lo[a], b.hi[a]), 0.5f), nc[a]);
+        }
+        int my_slot = -1;
+        unsigned free_slots = 0xFFu;
+        for (int round = 0; round < 8; ++round) {
+            float best = FLT_MAX;
+            int who = 64;  // slot * 8 + lane
+            if (has && my_slot < 0) {
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    const float cost = __fadd_rn(__fadd_rn((q & 4) ? -cc[0] : cc[0], (q & 2) ? -cc[1] : cc[1]),
+                                                 (q & 1) ? -cc[2] : cc[2]);
+                    if (((free_slots >> q) & 1u) && cost < best) {
+                        best = cost;
+                        who = q * 8 + c;
+                    }
                 }
-                if (x < 0) {
-                    const int64_t ref = key_tri(k, ~x, idx_mask);
-                    const int64_t tri = ref_tri ? (int64_t)ref_tri[ref] : ref;
-                    const int64_t slot = (int64_t)tbase + leaf_tris;
-                    const int32_t* ti = tidx + 3 * tri;
-                    woopify_dev(vtx(tv, ti[0]), vtx(tv, ti[1]), vtx(tv, ti[2]), woop + 3 * slot);
-                    prim[3 * slot] = (int32_t)tri;
-                    prim[3 * slot + 1] = -1;
-                    prim[3 * slot + 2] = -1;
-                    ++leaf_tris;
-                } else {
-                    st[sp++] = nodes[x].right;
-                    st[sp++] = nodes[x].left;
+            }
+            for (int m = 4; m > 0; m >>= 1) {
+                const float b2 = __shfl_xor_sync(kWarpAll, best, m);
+                const int w2 = __shfl_xor_sync(kWarpAll, who, m);
+                if (b2 < best || (b2 == best && w2 < who)) {
+                    best = b2;
+                    who = w2;
+                }
+            }
+            if (who < 64) {
+                free_slots &= ~(1u << (who >> 3));
+                if ((who & 7) == c) my_slot = who >> 3;
+            }
+            if (!__any_sync(kWarpAll, who < 64)) break;
+        }
+        // ---- per-axis exponent, grown while a child's upper bound does not fit a byte
+        int e[3];
+        for (int a = 0; a < 3; ++a) {
+            const float r = ceilf(log2f((hi[a] - lo[a]) / 255.0f));
+            e[a] = isfinite(r) ? (int)fmaxf(-127.f, fminf(127.f, r)) : 0;
+            for (;;) {
+                const float scale = ldexpf(1.0f, e[a]);
+                const bool over = has && (int)ceilf((b.hi[a] - lo[a]) / scale) > 255;
+                const bool grow = octet(over) != 0u && e[a] < 127;
+                if (grow) ++e[a];
+                if (!__any_sync(kWarpAll, grow)) break;
+            }
+        }
+        // ---- allocations: inner children as one block, leaf triangles as one
+        // run, taken for the warp's four nodes by one atomic
+        const bool inner = has && b.count > 3, leaf = has && !inner;
+        const unsigned n_inner = __popc(octet(inner));
+        unsigned n_tris = leaf ? (unsigned)b.count : 0u;
+        for (int m = 4; m > 0; m >>= 1) n_tris += __shfl_xor_sync(kWarpAll, n_tris, m);
+        const unsigned long long want = ((unsigned long long)n_tris << 32) | n_inner;
+        unsigned long long before = 0ull, total = 0ull;
+        for (int q = 0; q < 4; ++q) {
+            const unsigned long long x = __shfl_sync(kWarpAll, want, 8 * q);
+            if (q < (int)(shift >> 3)) before += x;
+            total += x;
+        }
+        unsigned long long got = 0ull;
+        if (lane == 0 && total) got = atomicAdd(&lv->alloc[level + 1], total);
+        got = __shfl_sync(kWarpAll, got, 0) + before;
+        const unsigned qbase = (unsigned)got;
+        const unsigned base = next0 + qbase, tbase = tri0 + (unsigned)(got >> 32);
+        if (active && !err && ((uint64_t)base + n_inner > node_cap || (uint64_t)tbase + n_tris > tri_cap)) err = 1u;
+        err = all_or(err);  // of the group
+        const bool go = active && err == 0u;
+        // ---- the node
+        const bool placed = has && my_slot >= 0;
+        const unsigned imask = all_or(placed && inner ? 1u << my_slot : 0u);
+        const unsigned counts = all_or(placed && leaf ? (unsigned)b.count << (2 * my_slot) : 0u);
+        const unsigned below = placed ? counts & ((1u << (2 * my_slot)) - 1u) : 0u;
+        const unsigned first_tri = __popc(below & 0x5555u) + 2u * __popc(below & 0xAAAAu);
+        const unsigned all_tris = __popc(counts & 0x5555u) + 2u * __popc(counts & 0xAAAAu);
+        if (c < 5) node_smem[group][c] = make_float4(0.f, 0.f, 0.f, 0.f);
+        __syncwarp();
+        unsigned char* bytes = reinterpret_cast<unsigned char*>(node_smem[group]);
+        if (go && c == 0) {
+            node_smem[group][0] = make_float4(lo[0], lo[1], lo[2],
+                                              __uint_as_float(((unsigned)e[0] & 0xFFu) | (((unsigned)e[1] & 0xFFu) << 8) |
+                                                              (((unsigned)e[2] & 0xFFu) << 16) | (imask << 24)));
+            reinterpret_cast<uint2*>(bytes)[2] = make_uint2(imask ? base : 0u, all_tris ? tbase : 0u);
+        }
+        if (go && placed) {
+            for (int a = 0; a < 3; ++a) {
+                const float scale = ldexpf(1.0f, e[a]);
+                bytes[32 + my_slot + 8 * a] = (uint8_t)(int)floorf((b.lo[a] - lo[a]) / scale);
+                bytes[32 + my_slot + 8 * (3 + a)] = (uint8_t)(int)ceilf((b.hi[a] - lo[a]) / scale);
+            }
+            if (inner) {
+                const unsigned rank = __popc(imask & ((1u << my_slot) - 1u));
+                bytes[24 + my_slot] = (uint8_t)((1u << 5) | (24u + my_slot));
+                next[qbase + rank] = Item{code, (int32_t)(base + rank)};
+            } else {
+                const uint32_t unary = b.count == 1 ? 1u : (b.count == 2 ? 3u : 7u);
+                bytes[24 + my_slot] = (uint8_t)((unary << 5) | (first_tri & 31u));
+                // the child's triangles, left first: a leaf, or a subtree of at most 3
+                int32_t st[4];
+                int sp = 0;
+                unsigned t = 0;
+                st[sp++] = code;
+                while (sp > 0) {
+                    const int32_t x = st[--sp];
+                    if (t >= (unsigned)b.count || (x >= 0 && sp + 2 > 4)) {  // counts disagree with the tree
+                        err = 2u;
+                        break;
+                    }
+                    if (x < 0) {
+                        const int64_t ref = key_tri(k, ~x, idx_mask);
+                        const int64_t slot = 3 * ((int64_t)tbase + first_tri + t);
+                        prim[slot] = ref_tri ? ref_tri[ref] : (int32_t)ref;
+                        ++t;
+                    } else {
+                        st[sp++] = nodes[x].right;
+                        st[sp++] = nodes[x].left;
+                    }
                 }
             }
         }
+        __syncwarp();
+        if (go && c < 5) out_nodes[(int64_t)it.addr * 5 + c] = node_smem[group][c];
+        if (err) atomicOr(&lv->error, err);
+        __syncwarp();
     }
-    float* nf = reinterpret_cast<float*>(bytes);
-    nf[0] = lo[0];
-    nf[1] = lo[1];
-    nf[2] = lo[2];
-    bytes[12] = (uint8_t)(int8_t)e[0];
-    bytes[13] = (uint8_t)(int8_t)e[1];
-    bytes[14] = (uint8_t)(int8_t)e[2];
-    bytes[15] = imask;
-    reinterpret_cast<int32_t*>(bytes)[4] = inner ? (int32_t)base : 0;
-    reinterpret_cast<int32_t*>(bytes)[5] = leaf_tris ? (int32_t)tbase : 0;
-    for (int q = 0; q < 5; ++q) out_nodes[(int64_t)it.addr * 5 + q] = node[q];
+}
+
+// Woop rows of the stored triangles, a thread each (prim: the triangle of
+// each slot's first row, -1 in a slot nothing took).
+__global__ void woop_rows_kernel(int64_t n, const float* v, const int32_t* idx, float4* woop, const int32_t* prim) {
+    const int64_t slot = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (slot >= n) return;
+    const int32_t tri = prim[3 * slot];
+    if (tri < 0) {
+        woop[3 * slot] = woop[3 * slot + 1] = woop[3 * slot + 2] = make_float4(0.f, 0.f, 0.f, 0.f);
+        return;
+    }
+    const int32_t* ti = idx + 3 * (int64_t)tri;
+    float4 rows[3];
+    woopify_dev(vtx(v, ti[0]), vtx(v, ti[1]), vtx(v, ti[2]), rows);
+    for (int q = 0; q < 3; ++q) woop[3 * slot + q] = rows[q];
 }
 
 unsigned blocks_of(int64_t n, int b) { return (unsigned)std::max<int64_t>(1, (n + b - 1) / b); }
@@ -1218,47 +1314,54 @@ unsigned blocks_of(int64_t n, int b) { return (unsigned)std::max<int64_t>(1, (n 
 // does not.  Node numbers come from prefix sums, counting down from n - 2 in
 // position order, so the last merge is the root (node 0) and the tree does
 // not depend on thread scheduling.
+//
+// A round is three launches over tiles of kPlocTile clusters: the nearest
+// neighbours of a tile and of the kPlocRadius clusters either side of it (so
+// that a tile knows its mutual pairs), with the tile's numbers of merges and
+// survivors; one block that sums those over the tiles; and the merge, which
+// writes the survivors and merged clusters to the other buffer.  Cluster
+// counts stay on the device and rounds are queued ahead of them.  Once
+// kPlocLast clusters or fewer are left, most of the rounds but little of the
+// work, one block does the remaining rounds in shared memory.  A cluster
+// carries its box, cost and count, so a merge reads nothing of the tree.
+// 500,000-triangle heightfield, 51 rounds: 1,320 us of kernels with two scans
+// and two copies to the host in every round -> 580 us and five copies.
 constexpr int kPlocRadius = 16;
+constexpr int kPlocTile = 256;
+constexpr int kPlocLast = 2048;
+constexpr int kPlocRoundsAhead = 6;
 
-struct CBox {
-    float lo[3], hi[3];
+struct PlocState {
+    int32_t m;      // clusters
+    int32_t top;    // next node number (counting down)
+    int32_t cur;    // buffer holding the clusters
+    uint32_t error; // a round that merged nothing (non-finite boxes)
+};
+struct Clusters {
+    int32_t* code[2];
+    NodeBox* box[2];
 };
 
-__device__ inline float merged_area(const CBox& a, const CBox& b) {
-    float lo[3], hi[3];
-    for (int q = 0; q < 3; ++q) {
-        lo[q] = fminf(a.lo[q], b.lo[q]);
-        hi[q] = fmaxf(a.hi[q], b.hi[q]);
-    }
-    return half_area(lo, hi);
-}
-
-__global__ void ploc_init_kernel(const uint64_t* k, uint64_t idx_mask, int64_t n, const float* v, const int32_t* idx,
-                                 int32_t* code, CBox* box) {
-    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    code[p] = ~(int32_t)p;
-    tri_box(v, idx, key_tri(k, p, idx_mask), box[p].lo, box[p].hi);
-}
-
-// Nearest neighbour of each cluster within the radius: least merged area,
-// ties to the nearer position, then to the cluster's partner i ^ 1, then to
-// the lower position.  The rule is the same seen from both sides of a pair,
-// and clusters with identical boxes (duplicated geometry) pair off with
-// their partners, half of them merging per round instead of one pair.
-__global__ void ploc_nn_kernel(const CBox* box, int64_t m, int32_t* nn) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m) return;
-    const CBox bi = box[i];
-    const int64_t j0 = i - kPlocRadius < 0 ? 0 : i - kPlocRadius;
-    const int64_t j1 = i + kPlocRadius >= m ? m - 1 : i + kPlocRadius;
+// Nearest neighbour of cluster i within the radius: least merged area, ties
+// to the nearer position, then to the cluster's partner i ^ 1, then to the
+// lower position.  The rule is the same seen from both sides of a pair, and
+// clusters with identical boxes (duplicated geometry) pair off with their
+// partners, half of them merging per round instead of one pair.
+template <class GetBox>
+__device__ inline int ploc_nearest(int i, int m, const NodeBox& bi, GetBox box) {
+    const int j0 = i - kPlocRadius < 0 ? 0 : i - kPlocRadius;
+    const int j1 = i + kPlocRadius >= m ? m - 1 : i + kPlocRadius;
     float best = FLT_MAX;
-    int64_t bj = i == 0 ? 1 : i - 1, bdist = INT64_MAX;
+    int bj = i == 0 ? 1 : i - 1, bdist = INT32_MAX;
     bool bpartner = false;
-    for (int64_t j = j0; j <= j1; ++j) {
+    for (int j = j0; j <= j1; ++j) {
         if (j == i) continue;
-        const float d = merged_area(bi, box[j]);
-        const int64_t dist = j > i ? j - i : i - j;
+        float4 l, h;
+        box(j, l, h);
+        const float lo[3] = {fminf(bi.lo[0], l.x), fminf(bi.lo[1], l.y), fminf(bi.lo[2], l.z)};
+        const float hi[3] = {fmaxf(bi.hi[0], h.x), fmaxf(bi.hi[1], h.y), fmaxf(bi.hi[2], h.z)};
+        const float d = half_area(lo, hi);
+        const int dist = j > i ? j - i : i - j;
         const bool partner = j == (i ^ 1);
         // ascending j: among full ties the first is the lowest position
         if (d < best || (d == best && (dist < bdist || (dist == bdist && partner && !bpartner)))) {
@@ -1268,64 +1371,261 @@ __global__ void ploc_nn_kernel(const CBox* box, int64_t m, int32_t* nn) {
             bpartner = partner;
         }
     }
-    nn[i] = (int32_t)bj;
+    return bj;
 }
 
-// merge[i] = 1 for the lower cluster of a mutual pair; keep[i] = 0 for the
-// upper one (it is absorbed).  Both arrays have an extra zero at m for the
-// scans' totals.
-__global__ void ploc_flags_kernel(const int32_t* nn, int64_t m, int32_t* merge, int32_t* keep) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i > m) return;
-    if (i == m) {
-        merge[i] = 0;
-        keep[i] = 0;
+// A cluster's part in a round.
+constexpr uint8_t kPlocMerges = 0x40;    // lower cluster of a mutual pair
+constexpr uint8_t kPlocAbsorbed = 0x80;  // upper one; low six bits: neighbour - cluster + kPlocRadius
+
+__global__ void ploc_init_kernel(int64_t n, const NodeBox* leaves, Clusters cl, PlocState* st) {
+    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (p == 0) st[0] = PlocState{(int32_t)n, (int32_t)(n - 2), 0, 0u};
+    if (p >= n) return;
+    cl.code[0][p] = ~(int32_t)p;
+    store_box(&cl.box[0][p], child_box(nullptr, leaves, ~(int32_t)p));
+}
+
+__device__ inline bool ploc_idle(const PlocState& s) { return s.error || s.m <= kPlocLast; }
+
+__global__ void __launch_bounds__(kPlocTile + 2 * kPlocRadius) ploc_pairs_kernel(Clusters cl, const PlocState* st,
+                                                                                 uint8_t* part, uint2* sums) {
+    constexpr int kReach = 2 * kPlocRadius;
+    __shared__ float4 slo[kPlocTile + 2 * kReach], shi[kPlocTile + 2 * kReach];
+    __shared__ int snn[kPlocTile + 2 * kPlocRadius];
+    __shared__ unsigned counts[2];
+    const PlocState s = *st;
+    const int t0 = blockIdx.x * kPlocTile;
+    if (ploc_idle(s) || t0 >= s.m) return;
+    const NodeBox* box = cl.box[s.cur];
+    for (int q = threadIdx.x; q < kPlocTile + 2 * kReach; q += blockDim.x) {
+        const int j = t0 - kReach + q;
+        if (j < 0 || j >= s.m) continue;
+        const float4* p = reinterpret_cast<const float4*>(box + j);
+        slo[q] = p[0];
+        shi[q] = p[1];
+    }
+    if (threadIdx.x < 2) counts[threadIdx.x] = 0u;
+    __syncthreads();
+    const int i = t0 - kPlocRadius + (int)threadIdx.x;
+    int nn = -1;
+    if (i >= 0 && i < s.m) {
+        const float4 l = slo[threadIdx.x + kPlocRadius], h = shi[threadIdx.x + kPlocRadius];
+        NodeBox bi;
+        bi.lo[0] = l.x; bi.lo[1] = l.y; bi.lo[2] = l.z;
+        bi.hi[0] = h.x; bi.hi[1] = h.y; bi.hi[2] = h.z;
+        nn = ploc_nearest(i, s.m, bi, [&](int j, float4& jl, float4& jh) {
+            jl = slo[j - t0 + kReach];
+            jh = shi[j - t0 + kReach];
+        });
+    }
+    snn[threadIdx.x] = nn;
+    __syncthreads();
+    bool merges = false, keeps = false;
+    if (i >= t0 && i < t0 + kPlocTile && i < s.m) {
+        const bool mutual = snn[nn - t0 + kPlocRadius] == i;
+        merges = mutual && i < nn;
+        const bool absorbed = mutual && i > nn;
+        keeps = !absorbed;
+        part[i] = (uint8_t)((nn - i + kPlocRadius) | (merges ? kPlocMerges : 0) | (absorbed ? kPlocAbsorbed : 0));
+    }
+    const unsigned bm = __ballot_sync(kWarpAll, merges), bk = __ballot_sync(kWarpAll, keeps);
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(&counts[0], (unsigned)__popc(bm));
+        atomicAdd(&counts[1], (unsigned)__popc(bk));
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) sums[blockIdx.x] = make_uint2(counts[0], counts[1]);
+}
+
+// Exclusive sums of the tiles' counts, and the state of the next round.
+__global__ void __launch_bounds__(1024) ploc_scan_kernel(const PlocState* st, PlocState* st_next, uint2* sums) {
+    __shared__ uint2 warp_sum[32];
+    const PlocState s = *st;
+    if (ploc_idle(s)) {
+        if (threadIdx.x == 0) *st_next = s;
         return;
     }
-    const int32_t j = nn[i];
-    const bool mutual = nn[j] == (int32_t)i;
-    merge[i] = mutual && (int32_t)i < j;
-    keep[i] = !(mutual && (int32_t)i > j);
+    const int tiles = (s.m + kPlocTile - 1) / kPlocTile;
+    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    uint2 carry = make_uint2(0u, 0u);
+    for (int t = 0; t < tiles; t += 1024) {
+        const int q = t + (int)threadIdx.x;
+        const uint2 own = q < tiles ? sums[q] : make_uint2(0u, 0u);
+        uint2 x = own;
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned a = __shfl_up_sync(kWarpAll, x.x, o), b = __shfl_up_sync(kWarpAll, x.y, o);
+            if (lane >= (unsigned)o) { x.x += a; x.y += b; }
+        }
+        if (lane == 31u) warp_sum[warp] = x;
+        __syncthreads();
+        if (warp == 0) {
+            uint2 y = warp_sum[lane];
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned a = __shfl_up_sync(kWarpAll, y.x, o), b = __shfl_up_sync(kWarpAll, y.y, o);
+                if (lane >= (unsigned)o) { y.x += a; y.y += b; }
+            }
+            warp_sum[lane] = y;
+        }
+        __syncthreads();
+        uint2 before = carry;
+        if (warp > 0) { before.x += warp_sum[warp - 1].x; before.y += warp_sum[warp - 1].y; }
+        if (q < tiles) sums[q] = make_uint2(before.x + x.x - own.x, before.y + x.y - own.y);
+        carry.x += warp_sum[31].x;
+        carry.y += warp_sum[31].y;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        PlocState n = s;
+        const int32_t merges = (int32_t)carry.x, kept = (int32_t)carry.y;
+        if (merges <= 0 || kept != s.m - merges || s.top - merges + 1 < 0) {
+            n.error = 1u;
+        } else {
+            n.m = kept;
+            n.top = s.top - merges;
+            n.cur = s.cur ^ 1;
+        }
+        *st_next = n;
+    }
 }
 
-__global__ void ploc_merge_kernel(const int32_t* nn, const int32_t* merge, const int32_t* rank, int64_t m, int64_t top,
-                                  const uint64_t* k, uint64_t idx_mask, const float* v, const int32_t* idx,
-                                  int32_t* code, CBox* box, BNode* nodes, int32_t* leaf_parent) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m || !merge[i]) return;
-    const int32_t j = nn[i];
-    const int32_t node = (int32_t)(top - rank[i]);
-    const int32_t c[2] = {code[i], code[j]};
-    float clo[2][3], chi[2][3], cc[2];
-    int32_t cn[2];
-    for (int q = 0; q < 2; ++q) child_box(nodes, k, idx_mask, v, idx, c[q], clo[q], chi[q], cn[q], &cc[q]);
-    BNode& nd = nodes[node];
-    nd.left = c[0];
-    nd.right = c[1];
-    nd.parent = -1;
-    nd.count = cn[0] + cn[1];
-    CBox u;
-    for (int a = 0; a < 3; ++a) {
-        u.lo[a] = fminf(clo[0][a], clo[1][a]);
-        u.hi[a] = fmaxf(chi[0][a], chi[1][a]);
-        nd.lo[a] = u.lo[a];
-        nd.hi[a] = u.hi[a];
-    }
-    nd.cost = node_cost(half_area(u.lo, u.hi), cc[0], cc[1]);
-    for (int q = 0; q < 2; ++q) {
-        if (c[q] >= 0) nodes[c[q]].parent = node;
-        else leaf_parent[~c[q]] = node;
-    }
-    code[i] = node;
-    box[i] = u;
+// A merged pair becomes node `node`.
+__device__ inline void ploc_link(BNode* nodes, int32_t node, int32_t left, int32_t right,
+                                 const NodeBox& b) {
+    *reinterpret_cast<int4*>(&nodes[node]) = make_int4(left, right, -1, 0);
+    store_box(&nodes[node].b, b);
+}
+__device__ inline void ploc_set_parent(BNode* nodes, int32_t* leaf_parent, int32_t code, int32_t node) {
+    if (code >= 0) nodes[code].parent = node;
+    else leaf_parent[~code] = node;
 }
 
-__global__ void ploc_compact_kernel(const int32_t* keep, const int32_t* pos, int64_t m, const int32_t* code,
-                                    const CBox* box, int32_t* code2, CBox* box2) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m || !keep[i]) return;
-    code2[pos[i]] = code[i];
-    box2[pos[i]] = box[i];
+__global__ void __launch_bounds__(kPlocTile) ploc_merge_kernel(Clusters cl, const PlocState* st, const PlocState* st_next,
+                                                               const uint8_t* part, const uint2* sums, BNode* nodes,
+                                                               int32_t* leaf_parent) {
+    __shared__ uint2 warp_sum[kPlocTile / 32];
+    const PlocState s = *st;
+    const int i = blockIdx.x * kPlocTile + threadIdx.x;
+    if (ploc_idle(s) || st_next->error || blockIdx.x * kPlocTile >= s.m) return;
+    const uint8_t f = i < s.m ? part[i] : kPlocAbsorbed;
+    const bool merges = (f & kPlocMerges) != 0, keeps = (f & kPlocAbsorbed) == 0;
+    const unsigned bm = __ballot_sync(kWarpAll, merges), bk = __ballot_sync(kWarpAll, keeps);
+    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, below = (1u << lane) - 1u;
+    if (lane == 0) warp_sum[warp] = make_uint2(__popc(bm), __popc(bk));
+    __syncthreads();
+    uint2 at = sums[blockIdx.x];
+    for (unsigned q = 0; q < warp; ++q) { at.x += warp_sum[q].x; at.y += warp_sum[q].y; }
+    if (!keeps) return;
+    const int32_t node = s.top - (int32_t)(at.x + __popc(bm & below));
+    const unsigned to = at.y + __popc(bk & below);
+    const int32_t* code = cl.code[s.cur];
+    const NodeBox* box = cl.box[s.cur];
+    int32_t c = code[i];
+    NodeBox b = child_box(nullptr, box, ~i);
+    if (merges) {
+        const int j = i + (int)(f & 0x3Fu) - kPlocRadius;
+        const int32_t c2 = code[j];
+        b = join(b, child_box(nullptr, box, ~j));
+        ploc_link(nodes, node, c, c2, b);
+        ploc_set_parent(nodes, leaf_parent, c, node);
+        ploc_set_parent(nodes, leaf_parent, c2, node);
+        c = node;
+    }
+    cl.code[s.cur ^ 1][to] = c;
+    store_box(&cl.box[s.cur ^ 1][to], b);
+}
+
+// All rounds from kPlocLast clusters on, in one block.
+struct PlocLast {
+    float4 lo[2][kPlocLast], hi[2][kPlocLast];  // lo.w: cost, hi.w: count
+    int32_t code[2][kPlocLast];
+    int32_t nn[kPlocLast];
+    uint2 warp_sum[32];
+};
+
+__global__ void __launch_bounds__(1024) ploc_last_kernel(Clusters cl, PlocState* st, BNode* nodes,
+                                                         int32_t* leaf_parent) {
+    extern __shared__ __align__(16) unsigned char raw[];
+    PlocLast& t = *reinterpret_cast<PlocLast*>(raw);
+    const PlocState s = *st;
+    if (s.error || s.m > kPlocLast) return;
+    int m = s.m, top = s.top, cur = 0;
+    for (int q = threadIdx.x; q < m; q += blockDim.x) {
+        const float4* p = reinterpret_cast<const float4*>(&cl.box[s.cur][q]);
+        t.lo[0][q] = p[0];
+        t.hi[0][q] = p[1];
+        t.code[0][q] = cl.code[s.cur][q];
+    }
+    __syncthreads();
+    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, below = (1u << lane) - 1u;
+    uint32_t error = 0u;
+    while (m > 1) {
+        auto load = [&](int j, float4& l, float4& h) {
+            l = t.lo[cur][j];
+            h = t.hi[cur][j];
+        };
+        auto get = [&](int j) {
+            float4 l, h;
+            load(j, l, h);
+            NodeBox b;
+            b.lo[0] = l.x; b.lo[1] = l.y; b.lo[2] = l.z; b.cost = l.w;
+            b.hi[0] = h.x; b.hi[1] = h.y; b.hi[2] = h.z; b.count = __float_as_int(h.w);
+            return b;
+        };
+        for (int i = threadIdx.x; i < m; i += blockDim.x) t.nn[i] = ploc_nearest(i, m, get(i), load);
+        __syncthreads();
+        int merged = 0, kept = 0;
+        for (int i0 = 0; i0 < m; i0 += blockDim.x) {
+            const int i = i0 + (int)threadIdx.x;
+            bool merges = false, keeps = false;
+            int j = 0;
+            if (i < m) {
+                j = t.nn[i];
+                const bool mutual = t.nn[j] == i;
+                merges = mutual && i < j;
+                keeps = !(mutual && i > j);
+            }
+            const unsigned bm = __ballot_sync(kWarpAll, merges), bk = __ballot_sync(kWarpAll, keeps);
+            if (lane == 0) t.warp_sum[warp] = make_uint2(__popc(bm), __popc(bk));
+            __syncthreads();
+            uint2 x = t.warp_sum[lane];
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned a = __shfl_up_sync(kWarpAll, x.x, o), b = __shfl_up_sync(kWarpAll, x.y, o);
+                if (lane >= (unsigned)o) { x.x += a; x.y += b; }
+            }
+            const unsigned all_m = __shfl_sync(kWarpAll, x.x, 31), all_k = __shfl_sync(kWarpAll, x.y, 31);
+            const unsigned wm = __shfl_sync(kWarpAll, x.x, warp ? warp - 1 : 0);
+            const unsigned wk = __shfl_sync(kWarpAll, x.y, warp ? warp - 1 : 0);
+            if (keeps) {
+                const int32_t node = top - (merged + (int)(warp ? wm : 0u) + __popc(bm & below));
+                const int to = kept + (int)(warp ? wk : 0u) + __popc(bk & below);
+                int32_t c = t.code[cur][i];
+                NodeBox b = get(i);
+                if (merges && node >= 0) {
+                    const int32_t c2 = t.code[cur][j];
+                    b = join(b, get(j));
+                    ploc_link(nodes, node, c, c2, b);
+                    ploc_set_parent(nodes, leaf_parent, c, node);
+                    ploc_set_parent(nodes, leaf_parent, c2, node);
+                    c = node;
+                }
+                t.code[cur ^ 1][to] = c;
+                t.lo[cur ^ 1][to] = make_float4(b.lo[0], b.lo[1], b.lo[2], b.cost);
+                t.hi[cur ^ 1][to] = make_float4(b.hi[0], b.hi[1], b.hi[2], __int_as_float(b.count));
+            }
+            merged += (int)all_m;
+            kept += (int)all_k;
+            __syncthreads();
+        }
+        if (merged <= 0 || kept != m - merged || top - merged + 1 < 0) {  // uniform: every thread has the same sums
+            error = 1u;
+            break;
+        }
+        m = kept;
+        top -= merged;
+        cur ^= 1;
+    }
+    if (threadIdx.x == 0) *st = PlocState{m, top, s.cur, error};
 }
 
 }  // namespace
@@ -1333,78 +1633,75 @@ __global__ void ploc_compact_kernel(const int32_t* keep, const int32_t* pos, int
 
 using namespace rq;
 
-// PLOC rounds on the clusters of the sorted triangles: nodes, boxes, counts,
-// costs and parent links as the radix tree + bottom-up boxes give them.
-static rq_status ploc_tree(const uint64_t* keys_sorted, uint64_t idx_mask, int64_t n, const float* vertices,
-                           const int32_t* indices, BNode* bn, int32_t* leaf_parent, cudaStream_t s) {
-    int32_t *code = nullptr, *code2 = nullptr, *nn = nullptr, *merge = nullptr, *keep = nullptr, *rank = nullptr,
-            *pos = nullptr;
-    CBox *box = nullptr, *box2 = nullptr;
-    void* temp = nullptr;
-    size_t temp_bytes = 0;
-    rq_status st = RQ_OK;
-    auto ok = [&](cudaError_t e) {
-        if (e != cudaSuccess && st == RQ_OK) st = cuda_fail(e, "rq_build_scene_gpu (PLOC)");
-        return st == RQ_OK;
-    };
-    const int64_t n1 = n + 1;
-    if (ok(cudaMalloc(&code, n * sizeof(int32_t))) && ok(cudaMalloc(&code2, n * sizeof(int32_t))) &&
-        ok(cudaMalloc(&nn, n * sizeof(int32_t))) && ok(cudaMalloc(&merge, n1 * sizeof(int32_t))) &&
-        ok(cudaMalloc(&keep, n1 * sizeof(int32_t))) && ok(cudaMalloc(&rank, n1 * sizeof(int32_t))) &&
-        ok(cudaMalloc(&pos, n1 * sizeof(int32_t))) && ok(cudaMalloc(&box, n * sizeof(CBox))) &&
-        ok(cudaMalloc(&box2, n * sizeof(CBox))) &&
-        ok(cub::DeviceScan::ExclusiveSum(nullptr, temp_bytes, merge, rank, (int)n1, s)) &&
-        ok(cudaMalloc(&temp, std::max<size_t>(temp_bytes, 1)))) {
-        ploc_init_kernel<<<blocks_of(n, 256), 256, 0, s>>>(keys_sorted, idx_mask, n, vertices, indices, code, box);
-        ok(cudaGetLastError());
-        int64_t m = n, top = n - 2;
-        // Each round merges at least the globally closest pair in reach; a
-        // round that merges nothing (non-finite boxes) is an error.
-        for (int round = 0; st == RQ_OK && m > 1; ++round) {
-            if (round > 100000) {
-                st = RQ_ERR_BAD_SCENE;
-                break;
-            }
-            ploc_nn_kernel<<<blocks_of(m, 256), 256, 0, s>>>(box, m, nn);
-            ploc_flags_kernel<<<blocks_of(m + 1, 256), 256, 0, s>>>(nn, m, merge, keep);
-            ok(cudaGetLastError());
-            size_t tb = temp_bytes;
-            ok(cub::DeviceScan::ExclusiveSum(temp, tb, merge, rank, (int)(m + 1), s));
-            tb = temp_bytes;
-            ok(cub::DeviceScan::ExclusiveSum(temp, tb, keep, pos, (int)(m + 1), s));
-            int32_t totals[2] = {0, 0};
-            ok(cudaMemcpyAsync(&totals[0], rank + m, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-            ok(cudaMemcpyAsync(&totals[1], pos + m, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-            ok(cudaStreamSynchronize(s));
-            if (st != RQ_OK) break;
-            const int64_t merges = totals[0], kept = totals[1];
-            if (merges <= 0 || kept != m - merges || top - merges + 1 < 0) {
-                st = RQ_ERR_BAD_SCENE;
-                break;
-            }
-            ploc_merge_kernel<<<blocks_of(m, 256), 256, 0, s>>>(nn, merge, rank, m, top, keys_sorted, idx_mask,
-                                                                vertices, indices, code, box, bn, leaf_parent);
-            ploc_compact_kernel<<<blocks_of(m, 256), 256, 0, s>>>(keep, pos, m, code, box, code2, box2);
-            ok(cudaGetLastError());
-            std::swap(code, code2);
-            std::swap(box, box2);
-            top -= merges;
-            m = kept;
-        }
-        if (st == RQ_OK && top != -1) st = RQ_ERR_BAD_SCENE;  // n - 1 nodes, the root last (node 0)
+// One device allocation cut into aligned buffers: laid out first, then made.
+struct Arena {
+    char* base = nullptr;
+    size_t bytes = 0;
+    std::vector<std::pair<void**, size_t>> parts;
+    template <class T>
+    void add(T** p, int64_t count) {
+        parts.emplace_back((void**)p, bytes);
+        bytes += ((size_t)std::max<int64_t>(1, count) * sizeof(T) + 255) / 256 * 256;
     }
-    ok(cudaStreamSynchronize(s));
-    cudaFree(code);
-    cudaFree(code2);
-    cudaFree(nn);
-    cudaFree(merge);
-    cudaFree(keep);
-    cudaFree(rank);
-    cudaFree(pos);
-    cudaFree(box);
-    cudaFree(box2);
-    cudaFree(temp);
-    return st;
+    cudaError_t make() {
+        const cudaError_t e = cudaMalloc(&base, std::max<size_t>(bytes, 256));
+        if (e == cudaSuccess)
+            for (auto& p : parts) *p.first = base + p.second;
+        return e;
+    }
+    void release() {
+        cudaFree(base);
+        base = nullptr;
+    }
+};
+
+// Buffers of the PLOC rounds.
+struct PlocBuffers {
+    Clusters cl{};
+    uint8_t* part = nullptr;
+    uint2* sums = nullptr;
+    PlocState* state = nullptr;  // two, by the parity of the round
+    void layout(Arena& a, int64_t n) {
+        for (int q = 0; q < 2; ++q) {
+            a.add(&cl.code[q], n);
+            a.add(&cl.box[q], n);
+        }
+        a.add(&part, n);
+        a.add(&sums, (n + kPlocTile - 1) / kPlocTile);
+        a.add(&state, 2);
+    }
+};
+
+// PLOC rounds on the leaves of the sorted triangles: nodes, boxes, counts,
+// costs and parent links as the radix tree + bottom-up boxes give them.
+static rq_status ploc_tree(const PlocBuffers& p, int64_t n, const NodeBox* leaves, BNode* bn, int32_t* leaf_parent,
+                           cudaStream_t s) {
+    RQ_CUDA(cudaFuncSetAttribute(ploc_last_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PlocLast)));
+    ploc_init_kernel<<<blocks_of(n, 256), 256, 0, s>>>(n, leaves, p.cl, p.state);
+    RQ_CUDA(cudaGetLastError());
+    PlocState now{(int32_t)n, (int32_t)(n - 2), 0, 0u};
+    int parity = 0;
+    // A round merges at least the globally closest pair in reach (one that
+    // merges nothing sets the error), so the clusters run out.
+    for (int64_t round = 0; now.m > kPlocLast; round += kPlocRoundsAhead) {
+        if (round > 100000) return RQ_ERR_BAD_SCENE;
+        const unsigned tiles = blocks_of(now.m, kPlocTile);
+        for (int q = 0; q < kPlocRoundsAhead; ++q, parity ^= 1) {
+            ploc_pairs_kernel<<<tiles, kPlocTile + 2 * kPlocRadius, 0, s>>>(p.cl, p.state + parity, p.part, p.sums);
+            ploc_scan_kernel<<<1, 1024, 0, s>>>(p.state + parity, p.state + (parity ^ 1), p.sums);
+            ploc_merge_kernel<<<tiles, kPlocTile, 0, s>>>(p.cl, p.state + parity, p.state + (parity ^ 1), p.part, p.sums,
+                                                          bn, leaf_parent);
+        }
+        RQ_CUDA(cudaGetLastError());
+        RQ_CUDA(cudaMemcpyAsync(&now, p.state + parity, sizeof(now), cudaMemcpyDeviceToHost, s));
+        RQ_CUDA(cudaStreamSynchronize(s));
+        if (now.error) return RQ_ERR_BAD_SCENE;
+    }
+    ploc_last_kernel<<<1, 1024, sizeof(PlocLast), s>>>(p.cl, p.state + parity, bn, leaf_parent);
+    RQ_CUDA(cudaGetLastError());
+    RQ_CUDA(cudaMemcpyAsync(&now, p.state + parity, sizeof(now), cudaMemcpyDeviceToHost, s));
+    RQ_CUDA(cudaStreamSynchronize(s));
+    return now.error || now.m != 1 || now.top != -1 ? RQ_ERR_BAD_SCENE : RQ_OK;  // n - 1 nodes, the root last (node 0)
 }
 
 // The references of a pre-split mesh: the box mesh (2 corners per
@@ -1516,18 +1813,6 @@ extern "C" rq_status rq_build_scene_gpu(const float* vertices, int64_t nv, const
     const float* bv = rm.n ? rm.v : vertices;
     const int32_t* bi = rm.n ? rm.idx : indices;
     const int64_t n = rm.n ? rm.n : nt;
-    // device scratch
-    uint64_t *keys = nullptr, *keys_sorted = nullptr;
-    BNode* bn = nullptr;
-    int32_t *leaf_parent = nullptr, *arrivals = nullptr;
-    CollapseDP* dp = nullptr;
-    unsigned* ob = nullptr;
-    Item *qa = nullptr, *qb = nullptr;
-    Ctr* ctr = nullptr;
-    void* cub_temp = nullptr;
-    float4 *nodes = nullptr, *woop = nullptr;
-    int32_t* prim = nullptr;
-    size_t cub_bytes = 0;
     int idx_bits = 1;
     while ((1ll << idx_bits) < n) ++idx_bits;
     const uint64_t idx_mask = (1ull << idx_bits) - 1;
@@ -1539,106 +1824,125 @@ extern "C" rq_status rq_build_scene_gpu(const float* vertices, int64_t nv, const
         return st == RQ_OK;
     };
     const int64_t node_cap = std::max<int64_t>(1, n);  // an 8-wide node per binary node at most
-    const int64_t q_cap = node_cap;
     constexpr size_t kPad = 256;
-    if (ok(cudaMalloc(&keys, n * sizeof(uint64_t)), "rq_build_scene_gpu") &&
-        ok(cudaMalloc(&keys_sorted, n * sizeof(uint64_t)), "rq_build_scene_gpu") &&
-        ok(cudaMalloc(&bn, std::max<int64_t>(1, n - 1) * sizeof(BNode)), "rq_build_scene_gpu") &&
-        ok(cudaMalloc(&leaf_parent, n * sizeof(int32_t)), "rq_build_scene_gpu") &&
-        ok(cudaMalloc(&arrivals, std::max<int64_t>(1, n - 1) * sizeof(int32_t)), "rq_build_scene_gpu") &&
-        ok(cudaMalloc(&dp, std::max<int64_t>(1, n - 1) * sizeof(CollapseDP)), "rq_build_scene_gpu") &&
-        ok(cudaMalloc(&ob, 6 * sizeof(unsigned)), "rq_build_scene_gpu") &&
-        ok(cudaMalloc(&qa, q_cap * sizeof(Item)), "rq_build_scene_gpu") &&
-        ok(cudaMalloc(&qb, q_cap * sizeof(Item)), "rq_build_scene_gpu") &&
-        ok(cudaMalloc(&ctr, sizeof(Ctr)), "rq_build_scene_gpu") &&
+    // device scratch, one allocation
+    uint64_t *keys = nullptr, *keys_sorted = nullptr;
+    BNode* bn = nullptr;
+    NodeBox* leaves = nullptr;
+    int32_t *leaf_parent = nullptr, *arrivals = nullptr;
+    CollapseDP* dp = nullptr;
+    unsigned* ob = nullptr;
+    Item* queue[2] = {nullptr, nullptr};
+    Levels* lv = nullptr;
+    char* cub_temp = nullptr;
+    PlocBuffers ploc;
+    size_t cub_bytes = 0;
+    Arena arena;
+    // The keys hold the triangle numbers in order below the Morton codes, so a
+    // stable sort by the codes alone orders them.
+    ok(cub::DeviceRadixSort::SortKeys(nullptr, cub_bytes, keys, keys_sorted, (int)n, idx_bits, end_bit, s),
+       "rq_build_scene_gpu");
+    arena.add(&keys, n);
+    arena.add(&keys_sorted, n);
+    arena.add(&bn, n - 1);
+    arena.add(&leaves, n);
+    arena.add(&leaf_parent, n);
+    arena.add(&arrivals, n - 1);
+    arena.add(&dp, n - 1);
+    arena.add(&ob, 6);
+    arena.add(&queue[0], node_cap);
+    arena.add(&queue[1], node_cap);
+    arena.add(&lv, 1);
+    arena.add(&cub_temp, (int64_t)cub_bytes);
+    if (method == RQ_GPU_BUILD_PLOC) ploc.layout(arena, n);
+    float4 *nodes = nullptr, *woop = nullptr;
+    int32_t* prim = nullptr;
+    if (st == RQ_OK && ok(arena.make(), "rq_build_scene_gpu") &&
         ok(cudaMalloc(&nodes, node_cap * 80 + kPad), "rq_build_scene_gpu") &&
         ok(cudaMalloc(&woop, n * 48 + kPad), "rq_build_scene_gpu") &&
         ok(cudaMalloc(&prim, n * 12), "rq_build_scene_gpu")) {
         const unsigned init[6] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u, 0u};
         ok(cudaMemcpyAsync(ob, init, sizeof(init), cudaMemcpyHostToDevice, s), "rq_build_scene_gpu");
-        ok(cudaMemsetAsync(nodes, 0, node_cap * 80 + kPad, s), "rq_build_scene_gpu");
-        ok(cudaMemsetAsync(woop, 0, n * 48 + kPad, s), "rq_build_scene_gpu");
+        ok(cudaMemsetAsync(woop + 3 * n, 0, kPad, s), "rq_build_scene_gpu");
+        ok(cudaMemsetAsync(prim, 0xFF, n * 12, s), "rq_build_scene_gpu");
         ok(cudaMemsetAsync(arrivals, 0, std::max<int64_t>(1, n - 1) * sizeof(int32_t), s), "rq_build_scene_gpu");
-        ok(cudaMemsetAsync(ctr, 0, sizeof(Ctr), s), "rq_build_scene_gpu");
+        ok(cudaMemsetAsync(lv, 0, sizeof(Levels), s), "rq_build_scene_gpu");
     }
     if (st == RQ_OK) {
         centroid_bounds_kernel<<<std::min<unsigned>(blocks_of(n, 256), 4 * 148), 256, 0, s>>>(bv, bi, n, ob);
         morton_kernel<<<blocks_of(n, 256), 256, 0, s>>>(bv, bi, n, ob, axis_bits, idx_bits, keys);
         ok(cudaGetLastError(), "rq_build_scene_gpu");
-        ok(cub::DeviceRadixSort::SortKeys(nullptr, cub_bytes, keys, keys_sorted, (int)n, 0, end_bit, s),
+        ok(cub::DeviceRadixSort::SortKeys(cub_temp, cub_bytes, keys, keys_sorted, (int)n, idx_bits, end_bit, s),
            "rq_build_scene_gpu");
-        ok(cudaMalloc(&cub_temp, std::max<size_t>(cub_bytes, 1)), "rq_build_scene_gpu");
-        ok(cub::DeviceRadixSort::SortKeys(cub_temp, cub_bytes, keys, keys_sorted, (int)n, 0, end_bit, s),
-           "rq_build_scene_gpu");
+        leaf_boxes_kernel<<<blocks_of(n, 256), 256, 0, s>>>(keys_sorted, idx_mask, n, bv, bi, leaves);
+        ok(cudaGetLastError(), "rq_build_scene_gpu");
     }
-    int64_t levels = 0, n_nodes = 1;
+    int64_t n_nodes = 1;
     if (st == RQ_OK && n > 1) {
         if (method == RQ_GPU_BUILD_PLOC) {
-            st = ploc_tree(keys_sorted, idx_mask, n, bv, bi, bn, leaf_parent, s);
+            st = ploc_tree(ploc, n, leaves, bn, leaf_parent, s);
         } else {
             radix_tree_kernel<<<blocks_of(n - 1, 256), 256, 0, s>>>(keys_sorted, n, bn, leaf_parent);
-            boxes_kernel<<<blocks_of(n, 256), 256, 0, s>>>(keys_sorted, idx_mask, n, bv, bi, bn,
-                                                           leaf_parent, arrivals);
+            boxes_kernel<<<blocks_of(n, 256), 256, 0, s>>>(n, leaves, bn, leaf_parent, arrivals);
             ok(cudaGetLastError(), "rq_build_scene_gpu");
         }
         for (int pass = 0; pass < optimize_passes && st == RQ_OK; ++pass) {
             ok(cudaMemsetAsync(arrivals, 0, (n - 1) * sizeof(int32_t), s), "rq_build_scene_gpu");
             if (thread_treelets)
-                treelet_kernel<<<blocks_of(n, 128), 128, 0, s>>>(keys_sorted, idx_mask, n, bv, bi, bn,
-                                                                 leaf_parent, arrivals, kTreeletLeaves);
+                treelet_kernel<<<blocks_of(n, 128), 128, 0, s>>>(n, leaves, bn, leaf_parent, arrivals, kTreeletLeaves);
             else
                 treelet_warp_kernel<<<blocks_of(n, kTreeletWarpBlock), kTreeletWarpBlock, 0, s>>>(
-                    keys_sorted, idx_mask, n, bv, bi, bn, leaf_parent, arrivals, kTreeletLeaves);
+                    n, leaves, bn, leaf_parent, arrivals, kTreeletLeaves);
             ok(cudaGetLastError(), "rq_build_scene_gpu");
         }
         if (st == RQ_OK) {
             ok(cudaMemsetAsync(arrivals, 0, (n - 1) * sizeof(int32_t), s), "rq_build_scene_gpu");
-            collapse_dp_kernel<<<blocks_of(n, 256), 256, 0, s>>>(keys_sorted, idx_mask, n, bv, bi, bn,
-                                                                 leaf_parent, arrivals, dp);
+            collapse_dp_kernel<<<blocks_of(n, 256), 256, 0, s>>>(n, leaves, bn, leaf_parent, arrivals, dp);
             ok(cudaGetLastError(), "rq_build_scene_gpu");
         }
     }
     if (st == RQ_OK) {
         // level 0: the root (binary node 0, or the single triangle)
         const Item root{n > 1 ? 0 : ~0, 0};
-        const Ctr c0{1ull, 0ull, 0ull, 0u};
-        ok(cudaMemcpyAsync(qa, &root, sizeof(root), cudaMemcpyHostToDevice, s), "rq_build_scene_gpu");
-        ok(cudaMemcpyAsync(ctr, &c0, sizeof(c0), cudaMemcpyHostToDevice, s), "rq_build_scene_gpu");
-        int64_t n_items = 1;
-        while (st == RQ_OK && n_items > 0) {
-            expand_kernel<<<blocks_of(n_items, 128), 128, 0, s>>>(qa, n_items, qb, q_cap, bn, keys_sorted, idx_mask,
-                                                                  bv, bi, vertices, indices, rm.tri, nodes, node_cap,
-                                                                  woop, prim, n,
-                                                                  ctr, n > 1 ? dp : nullptr);
-            ok(cudaGetLastError(), "rq_build_scene_gpu");
-            Ctr c{};
-            ok(cudaMemcpyAsync(&c, ctr, sizeof(Ctr), cudaMemcpyDeviceToHost, s), "rq_build_scene_gpu");
-            ok(cudaStreamSynchronize(s), "rq_build_scene_gpu");
-            if (st != RQ_OK) break;
-            if (c.error) {
-                st = RQ_ERR_BAD_SCENE;  // capacity exceeded: cannot happen for a valid radix tree
+        const unsigned long long one = 1ull;
+        ok(cudaMemcpyAsync(queue[0], &root, sizeof(root), cudaMemcpyHostToDevice, s), "rq_build_scene_gpu");
+        ok(cudaMemcpyAsync(&lv->alloc[0], &one, sizeof(one), cudaMemcpyHostToDevice, s), "rq_build_scene_gpu");
+        // An 8-wide tree of n triangles: eight levels ahead are rarely too many.
+        constexpr int kAhead = 8;
+        const unsigned grid = std::min<unsigned>(blocks_of(node_cap, kExpandBlock / 8), 148 * 8);
+        unsigned error = 0u;
+        unsigned long long left = 1ull;
+        for (int level = 0; st == RQ_OK && left != 0;) {
+            if (level + kAhead > kMaxLevels) {
+                st = RQ_ERR_BAD_SCENE;
                 break;
             }
-            n_items = (int64_t)c.next;
-            n_nodes = (int64_t)c.nodes;
-            std::swap(qa, qb);
-            ok(cudaMemsetAsync(&ctr->next, 0, sizeof(unsigned long long), s), "rq_build_scene_gpu");
-            if (++levels > 4096) st = RQ_ERR_BAD_SCENE;
+            for (int q = 0; q < kAhead; ++q, ++level)
+                expand_kernel<<<grid, kExpandBlock, 0, s>>>(level, queue[level & 1], queue[(level + 1) & 1], bn, leaves,
+                                                            keys_sorted, idx_mask, rm.tri, nodes, (unsigned)node_cap, prim,
+                                                            (unsigned)n, lv, n > 1 ? dp : nullptr);
+            unsigned total = 0u;
+            ok(cudaGetLastError(), "rq_build_scene_gpu");
+            ok(cudaMemcpyAsync(&left, &lv->alloc[level], sizeof(left), cudaMemcpyDeviceToHost, s), "rq_build_scene_gpu");
+            ok(cudaMemcpyAsync(&total, &lv->node_base[level], sizeof(total), cudaMemcpyDeviceToHost, s),
+               "rq_build_scene_gpu");
+            ok(cudaMemcpyAsync(&error, &lv->error, sizeof(error), cudaMemcpyDeviceToHost, s), "rq_build_scene_gpu");
+            ok(cudaStreamSynchronize(s), "rq_build_scene_gpu");
+            left &= 0xFFFFFFFFull;
+            n_nodes = (int64_t)total + (int64_t)left;
+            if (st == RQ_OK && error) st = RQ_ERR_BAD_SCENE;  // capacity exceeded: cannot happen for a valid tree
+        }
+        if (st == RQ_OK) {
+            woop_rows_kernel<<<blocks_of(n, 128), 128, 0, s>>>(n, vertices, indices, woop, prim);
+            ok(cudaGetLastError(), "rq_build_scene_gpu");
+            ok(cudaMemsetAsync(nodes + 5 * n_nodes, 0, kPad, s), "rq_build_scene_gpu");
         }
     }
     float root[20] = {};
-    if (st == RQ_OK) ok(cudaMemcpy(root, nodes, sizeof(root), cudaMemcpyDeviceToHost), "rq_build_scene_gpu");
-    cudaFree(keys);
-    cudaFree(keys_sorted);
-    cudaFree(bn);
-    cudaFree(leaf_parent);
-    cudaFree(arrivals);
-    cudaFree(dp);
-    cudaFree(ob);
-    cudaFree(qa);
-    cudaFree(qb);
-    cudaFree(ctr);
-    cudaFree(cub_temp);
+    if (st == RQ_OK)
+        ok(cudaMemcpyAsync(root, nodes, sizeof(root), cudaMemcpyDeviceToHost, s), "rq_build_scene_gpu");
+    ok(cudaStreamSynchronize(s), "rq_build_scene_gpu");  // nothing reads the scratch any more
+    arena.release();
     rm.release();
     if (st != RQ_OK) {
         cudaFree(nodes);
