@@ -35,6 +35,8 @@
 #include <cfloat>
 #include <cmath>
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <utility>
 #include <vector>
 
@@ -1633,26 +1635,81 @@ __global__ void __launch_bounds__(1024) ploc_last_kernel(Clusters cl, PlocState*
 
 using namespace rq;
 
-// One device allocation cut into aligned buffers: laid out first, then made.
+// Where builds take their scratch from: a memory pool per device that keeps
+// up to kPoolKeepBytes between builds while a scene built on the device lives
+// (a new block of memory costs ~330 us to map and ~270 us to unmap, up to
+// several ms now and then; a build of 500,000 triangles takes 4 ms besides).
+// The memory goes back to the device with the last such scene.  A pool is
+// safe for any number of threads and streams, and hands a block that one
+// stream freed to another only in order.
+constexpr uint64_t kPoolKeepBytes = 256ull << 20;  // the scratch of about a million triangles
+
+struct ScratchPool {
+    std::mutex mu;
+    struct Device {
+        cudaMemPool_t pool = nullptr;
+        int users = 0;  // scenes built on the device and builds under way
+    };
+    std::map<int, Device> devices;
+
+    cudaError_t enter(int dev, cudaMemPool_t* pool) {
+        std::lock_guard<std::mutex> lk(mu);
+        Device& d = devices[dev];
+        if (!d.pool) {
+            cudaMemPoolProps props{};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = dev;
+            cudaError_t e = cudaMemPoolCreate(&d.pool, &props);
+            if (e != cudaSuccess) return e;
+            uint64_t keep = kPoolKeepBytes;
+            e = cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+            if (e != cudaSuccess) {
+                cudaMemPoolDestroy(d.pool);
+                d.pool = nullptr;
+                return e;
+            }
+        }
+        ++d.users;
+        *pool = d.pool;
+        return cudaSuccess;
+    }
+    void leave(int dev) {
+        std::lock_guard<std::mutex> lk(mu);
+        Device& d = devices[dev];
+        if (--d.users == 0) cudaMemPoolTrimTo(d.pool, 0);
+    }
+};
+static ScratchPool& scratch_pool() {
+    static ScratchPool* p = new ScratchPool();  // never destroyed: scenes may outlive static objects
+    return *p;
+}
+void rq::gpu_built_scene_gone(int device) { scratch_pool().leave(device); }
+
+// One allocation from the pool cut into aligned buffers: laid out first, then
+// made.
 struct Arena {
     char* base = nullptr;
     size_t bytes = 0;
+    cudaStream_t stream = nullptr;
     std::vector<std::pair<void**, size_t>> parts;
     template <class T>
     void add(T** p, int64_t count) {
         parts.emplace_back((void**)p, bytes);
         bytes += ((size_t)std::max<int64_t>(1, count) * sizeof(T) + 255) / 256 * 256;
     }
-    cudaError_t make() {
-        const cudaError_t e = cudaMalloc(&base, std::max<size_t>(bytes, 256));
+    cudaError_t make(cudaMemPool_t pool, cudaStream_t s) {
+        stream = s;
+        const cudaError_t e = cudaMallocFromPoolAsync((void**)&base, std::max<size_t>(bytes, 256), pool, s);
         if (e == cudaSuccess)
             for (auto& p : parts) *p.first = base + p.second;
         return e;
     }
     void release() {
-        cudaFree(base);
+        if (base) cudaFreeAsync(base, stream);
         base = nullptr;
     }
+    ~Arena() { release(); }
 };
 
 // Buffers of the PLOC rounds.
@@ -1711,71 +1768,61 @@ struct RefMesh {
     int32_t* idx = nullptr;
     int32_t* tri = nullptr;
     int64_t n = 0;
-    void release() {
-        cudaFree(v);
-        cudaFree(idx);
-        cudaFree(tri);
-        *this = RefMesh{};
-    }
+    Arena arena;
 };
 
 // Cuts the nt triangles into at most nt + nt * budget / 100 references
 // (fewer when few triangles waste box area).  Leaves rm.n = 0 when there is
 // nothing to split.  The indices have been checked.
-static rq_status presplit(const float* v, const int32_t* idx, int64_t nt, int budget, RefMesh& rm, cudaStream_t s) {
+static rq_status presplit(const float* v, const int32_t* idx, int64_t nt, int budget, RefMesh& rm, cudaMemPool_t pool,
+                          cudaStream_t s) {
     const int64_t extra = std::min<int64_t>((int64_t)((double)nt * budget / 100.0), (int64_t)INT32_MAX / 4 - nt);
     if (extra <= 0) return RQ_OK;
-    rq_status st = RQ_OK;
-    auto ok = [&](cudaError_t e) {
-        if (e != cudaSuccess && st == RQ_OK) st = cuda_fail(e, "rq_build_scene_gpu (split)");
-        return st == RQ_OK;
-    };
     unsigned* sb = nullptr;
     float *prio = nullptr, *sum = nullptr;
     int64_t *pieces = nullptr, *off = nullptr;
-    void* temp = nullptr;
+    char* temp = nullptr;
     size_t b_sum = 0, b_scan = 0;
-    int64_t refs = 0;
-    if (ok(cudaMalloc(&sb, 6 * sizeof(unsigned))) && ok(cudaMalloc(&prio, nt * sizeof(float))) &&
-        ok(cudaMalloc(&sum, sizeof(float))) && ok(cudaMalloc(&pieces, nt * sizeof(int64_t))) &&
-        ok(cudaMalloc(&off, nt * sizeof(int64_t))) &&
-        ok(cub::DeviceReduce::Sum(nullptr, b_sum, prio, sum, (int)nt, s)) &&
-        ok(cub::DeviceScan::ExclusiveSum(nullptr, b_scan, pieces, off, (int)nt, s)) &&
-        ok(cudaMalloc(&temp, std::max<size_t>({b_sum, b_scan, (size_t)1})))) {
-        const unsigned init[6] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u, 0u};
-        ok(cudaMemcpyAsync(sb, init, sizeof(init), cudaMemcpyHostToDevice, s));
-        scene_bounds_kernel<<<std::min<unsigned>(blocks_of(nt, 256), 4 * 148), 256, 0, s>>>(v, idx, nt, sb);
-        split_priority_kernel<<<blocks_of(nt, 256), 256, 0, s>>>(v, idx, nt, sb, prio);
-        ok(cudaGetLastError());
-        ok(cub::DeviceReduce::Sum(temp, b_sum, prio, sum, (int)nt, s));
-        split_count_kernel<<<blocks_of(nt, 256), 256, 0, s>>>(prio, nt, sum, (double)extra, pieces);
-        ok(cudaGetLastError());
-        ok(cub::DeviceScan::ExclusiveSum(temp, b_scan, pieces, off, (int)nt, s));
-        int64_t tail[2] = {0, 0};
-        ok(cudaMemcpyAsync(&tail[0], off + nt - 1, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-        ok(cudaMemcpyAsync(&tail[1], pieces + nt - 1, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-        ok(cudaStreamSynchronize(s));
-        refs = tail[0] + tail[1];
-        if (st == RQ_OK && (refs < nt || refs > (int64_t)INT32_MAX / 4)) st = RQ_ERR_INVALID_ARG;
+    RQ_CUDA(cub::DeviceReduce::Sum(nullptr, b_sum, prio, sum, (int)nt, s));
+    RQ_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, b_scan, pieces, off, (int)nt, s));
+    Arena arena;  // freed in stream order, after the kernels that read it
+    arena.add(&sb, 6);
+    arena.add(&prio, nt);
+    arena.add(&sum, 1);
+    arena.add(&pieces, nt);
+    arena.add(&off, nt);
+    arena.add(&temp, (int64_t)std::max(b_sum, b_scan));
+    RQ_CUDA(arena.make(pool, s));
+    const unsigned init[6] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u, 0u};
+    RQ_CUDA(cudaMemcpyAsync(sb, init, sizeof(init), cudaMemcpyHostToDevice, s));
+    scene_bounds_kernel<<<std::min<unsigned>(blocks_of(nt, 256), 4 * 148), 256, 0, s>>>(v, idx, nt, sb);
+    split_priority_kernel<<<blocks_of(nt, 256), 256, 0, s>>>(v, idx, nt, sb, prio);
+    RQ_CUDA(cudaGetLastError());
+    RQ_CUDA(cub::DeviceReduce::Sum(temp, b_sum, prio, sum, (int)nt, s));
+    split_count_kernel<<<blocks_of(nt, 256), 256, 0, s>>>(prio, nt, sum, (double)extra, pieces);
+    RQ_CUDA(cudaGetLastError());
+    RQ_CUDA(cub::DeviceScan::ExclusiveSum(temp, b_scan, pieces, off, (int)nt, s));
+    int64_t tail[2] = {0, 0};
+    RQ_CUDA(cudaMemcpyAsync(&tail[0], off + nt - 1, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+    RQ_CUDA(cudaMemcpyAsync(&tail[1], pieces + nt - 1, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+    RQ_CUDA(cudaStreamSynchronize(s));
+    const int64_t refs = tail[0] + tail[1];
+    if (refs < nt || refs > (int64_t)INT32_MAX / 4) return RQ_ERR_INVALID_ARG;
+    if (refs > nt) {
+        rm.arena.add(&rm.v, refs * 6);
+        rm.arena.add(&rm.idx, refs * 3);
+        rm.arena.add(&rm.tri, refs);
+        RQ_CUDA(rm.arena.make(pool, s));
+        split_kernel<<<blocks_of(nt, 128), 128, 0, s>>>(v, idx, nt, sb, pieces, off, rm.v, rm.idx, rm.tri);
+        RQ_CUDA(cudaGetLastError());
+        rm.n = refs;
     }
-    if (st == RQ_OK && refs > nt) {
-        if (ok(cudaMalloc(&rm.v, refs * 6 * sizeof(float))) && ok(cudaMalloc(&rm.idx, refs * 3 * sizeof(int32_t))) &&
-            ok(cudaMalloc(&rm.tri, refs * sizeof(int32_t)))) {
-            split_kernel<<<blocks_of(nt, 128), 128, 0, s>>>(v, idx, nt, sb, pieces, off, rm.v, rm.idx, rm.tri);
-            ok(cudaGetLastError());
-            rm.n = refs;
-        }
-    }
-    if (st != RQ_OK) rm.release();
-    ok(cudaStreamSynchronize(s));  // the temporaries below are freed after the kernels that read them
-    cudaFree(sb);
-    cudaFree(prio);
-    cudaFree(sum);
-    cudaFree(pieces);
-    cudaFree(off);
-    cudaFree(temp);
-    return st;
+    return RQ_OK;
 }
+
+static rq_status build_scene(const float* vertices, int64_t nv, const int32_t* indices, int64_t nt, int method,
+                             int optimize_passes, int split_budget, rq_scene_t* out, cudaMemPool_t pool, int device,
+                             cudaStream_t s);
 
 extern "C" rq_status rq_build_scene_gpu(const float* vertices, int64_t nv, const int32_t* indices, int64_t nt,
                                         int method, int optimize_passes, int split_budget, rq_scene_t* out,
@@ -1785,27 +1832,42 @@ extern "C" rq_status rq_build_scene_gpu(const float* vertices, int64_t nv, const
     method &= ~RQ_GPU_BUILD_THREAD_TREELETS;
     if (method != RQ_GPU_BUILD_LBVH && method != RQ_GPU_BUILD_PLOC) return RQ_ERR_INVALID_ARG;
     if (split_budget < 0 || split_budget > 400) return RQ_ERR_INVALID_ARG;
-    cudaStream_t s = (cudaStream_t)stream;
+    int device = 0;
+    RQ_CUDA(cudaGetDevice(&device));
+    cudaMemPool_t pool = nullptr;
+    {
+        const cudaError_t e = scratch_pool().enter(device, &pool);
+        if (e != cudaSuccess) return cuda_fail(e, "rq_build_scene_gpu: scratch pool");
+    }
+    const rq_status st = build_scene(vertices, nv, indices, nt, method | (thread_treelets ? RQ_GPU_BUILD_THREAD_TREELETS : 0),
+                                     optimize_passes, split_budget, out, pool, device, (cudaStream_t)stream);
+    if (st != RQ_OK) scratch_pool().leave(device);  // otherwise the scene does, when it is destroyed
+    return st;
+}
+
+static rq_status build_scene(const float* vertices, int64_t nv, const int32_t* indices, int64_t nt, int method,
+                             int optimize_passes, int split_budget, rq_scene_t* out, cudaMemPool_t pool, int device,
+                             cudaStream_t s) {
+    const bool thread_treelets = (method & RQ_GPU_BUILD_THREAD_TREELETS) != 0;
+    method &= ~RQ_GPU_BUILD_THREAD_TREELETS;
     {
         // indices first: every kernel below reads vertices through them
         unsigned* bad_d = nullptr;
         unsigned bad = 0;
-        RQ_CUDA(cudaMalloc(&bad_d, sizeof(unsigned)));
-        cudaError_t e = cudaMemsetAsync(bad_d, 0, sizeof(unsigned), s);
-        if (e == cudaSuccess) {
-            check_indices_kernel<<<std::min<unsigned>(blocks_of(3 * nt, 256), 8 * 148), 256, 0, s>>>(
-                indices, 3 * nt, nv, bad_d);
-            e = cudaGetLastError();
-        }
-        if (e == cudaSuccess) e = cudaMemcpyAsync(&bad, bad_d, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        cudaFree(bad_d);
-        if (e != cudaSuccess) return cuda_fail(e, "rq_build_scene_gpu");
+        Arena arena;
+        arena.add(&bad_d, 1);
+        RQ_CUDA(arena.make(pool, s));
+        RQ_CUDA(cudaMemsetAsync(bad_d, 0, sizeof(unsigned), s));
+        check_indices_kernel<<<std::min<unsigned>(blocks_of(3 * nt, 256), 8 * 148), 256, 0, s>>>(indices, 3 * nt, nv,
+                                                                                                 bad_d);
+        RQ_CUDA(cudaGetLastError());
+        RQ_CUDA(cudaMemcpyAsync(&bad, bad_d, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+        RQ_CUDA(cudaStreamSynchronize(s));
         if (bad) return RQ_ERR_INVALID_ARG;
     }
     RefMesh rm;
     if (split_budget > 0) {
-        const rq_status ps = presplit(vertices, indices, nt, split_budget, rm, s);
+        const rq_status ps = presplit(vertices, indices, nt, split_budget, rm, pool, s);
         if (ps != RQ_OK) return ps;
     }
     // The tree stages read boxes from the box mesh when the triangles were
@@ -1855,12 +1917,17 @@ extern "C" rq_status rq_build_scene_gpu(const float* vertices, int64_t nv, const
     arena.add(&lv, 1);
     arena.add(&cub_temp, (int64_t)cub_bytes);
     if (method == RQ_GPU_BUILD_PLOC) ploc.layout(arena, n);
+    // the scene's buffers, one allocation of its own
+    char* block = nullptr;
+    const size_t node_bytes = ((size_t)node_cap * 80 + kPad + 255) / 256 * 256;
+    const size_t woop_bytes = ((size_t)n * 48 + kPad + 255) / 256 * 256;
     float4 *nodes = nullptr, *woop = nullptr;
     int32_t* prim = nullptr;
-    if (st == RQ_OK && ok(arena.make(), "rq_build_scene_gpu") &&
-        ok(cudaMalloc(&nodes, node_cap * 80 + kPad), "rq_build_scene_gpu") &&
-        ok(cudaMalloc(&woop, n * 48 + kPad), "rq_build_scene_gpu") &&
-        ok(cudaMalloc(&prim, n * 12), "rq_build_scene_gpu")) {
+    if (st == RQ_OK && ok(arena.make(pool, s), "rq_build_scene_gpu") &&
+        ok(cudaMalloc(&block, node_bytes + woop_bytes + (size_t)n * 12), "rq_build_scene_gpu")) {
+        nodes = (float4*)block;
+        woop = (float4*)(block + node_bytes);
+        prim = (int32_t*)(block + node_bytes + woop_bytes);
         const unsigned init[6] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u, 0u};
         ok(cudaMemcpyAsync(ob, init, sizeof(init), cudaMemcpyHostToDevice, s), "rq_build_scene_gpu");
         ok(cudaMemsetAsync(woop + 3 * n, 0, kPad, s), "rq_build_scene_gpu");
@@ -1941,18 +2008,16 @@ extern "C" rq_status rq_build_scene_gpu(const float* vertices, int64_t nv, const
     float root[20] = {};
     if (st == RQ_OK)
         ok(cudaMemcpyAsync(root, nodes, sizeof(root), cudaMemcpyDeviceToHost, s), "rq_build_scene_gpu");
-    ok(cudaStreamSynchronize(s), "rq_build_scene_gpu");  // nothing reads the scratch any more
-    arena.release();
-    rm.release();
+    ok(cudaStreamSynchronize(s), "rq_build_scene_gpu");
     if (st != RQ_OK) {
-        cudaFree(nodes);
-        cudaFree(woop);
-        cudaFree(prim);
+        cudaFree(block);
         return st;
     }
     rq_scene* sc = new rq_scene();
     sc->kind = RQ_BVH_CWBVH;
-    cudaGetDevice(&sc->device);
+    sc->device = device;
+    sc->block = block;
+    sc->gpu_built = true;
     sc->nodes = nodes;
     sc->woop = woop;
     sc->prim_index = prim;

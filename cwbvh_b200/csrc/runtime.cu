@@ -338,11 +338,14 @@ rq_status rq_scene_from_host_bvh(rq_host_bvh_t bvh, rq_scene_t* out) {
 
 rq_status rq_scene_destroy(rq_scene_t scene) {
     if (!scene) return RQ_ERR_INVALID_ARG;
-    if (scene->owned) {
+    if (scene->block) {
+        cudaFree(scene->block);
+    } else if (scene->owned) {
         cudaFree((void*)scene->nodes);
         cudaFree((void*)scene->woop);
         if (scene->prim_index) cudaFree((void*)scene->prim_index);
     }
+    if (scene->gpu_built) gpu_built_scene_gone(scene->device);
     delete scene;
     return RQ_OK;
 }
