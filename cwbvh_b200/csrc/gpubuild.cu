@@ -653,231 +653,255 @@ __global__ void treelet_kernel(int64_t n, const NodeBox* leaves, BNode* nodes, i
 // ---- The same restructuring with a warp per treelet (the parallel form of
 // Karras and Aila, section 4.2).  Lanes walk up the tree as in
 // treelet_kernel; at each step the nodes whose treelets are due are taken one
-// at a time by the whole warp: lane q holds leaf q while the treelet grows,
-// the subsets of one size are costed by different lanes (smaller subsets
-// first, so every partition's two parts are ready; a subset's box is its
-// box without its highest leaf, kept in shared memory, joined with that
-// leaf's), and the 63 partitions of the 7-leaf set are spread over the lanes
-// and reduced with shuffles.  Every subset's cost is the same expression in
-// the same order as in restructure(), and the chosen partition is the first
-// minimum in its enumeration order there, so the trees are identical.
+// at a time by the whole warp: lane q holds leaf q (its box and, ahead of its
+// being opened, its links) while the treelet grows; the subsets of one size
+// are costed by different lanes, smaller subsets first, so every partition's
+// two parts are ready; the 31 partitions of a 6-leaf set are spread over four
+// lanes and the 63 of the 7-leaf set over the warp; and a lane writes each
+// node of the new treelet.  Every subset's cost is the same expression as in
+// restructure(), over the same partitions (a subset's lowest leaf stays in P,
+// the others run down through the subsets of the rest), and the chosen
+// partition is the first minimum in its order there, so the trees are
+// identical.
+//
+// Bound by the warp's own chain of steps and, up the tree, by the chain of
+// treelets.  A lane's subsets are worked out once and kept in registers (a
+// table in constant memory costs a pass per lane), only partitions that hold
+// the lowest leaf are formed, and a subset's box is made from its leaves'
+// (two 16-byte reads each) so that the table is 1 KB and not 4 per warp.  Two
+// passes over 500,000 triangles: 2,854 -> TREELET_US us.
 constexpr unsigned kWarpAll = 0xFFFFFFFFu;
 
+struct TreeletSmem {
+    float4 lo[8], hi[8];  // leaf boxes
+    float cost[1 << kTreeletLeaves];
+    uint8_t part[1 << kTreeletLeaves];
+    int32_t leaf[8], count[8], inner[8];
+    int32_t set[8];  // the leaf set of each node of the new treelet
+};
+
+// The subsets of 7 leaves by lane: row 0 those of 2 leaves, rows 1-2 of 3 (35
+// of them), 3-4 of 4, 5 of 5, and 6 those of 6, each for four lanes; 0 where a
+// lane has none.
 struct SubsetTable {
-    uint8_t set[127];   // the subsets of 7 leaves by size, then value
-    uint8_t start[9];   // first entry of each size (start[8] = 127)
+    uint8_t set[7][32];
 };
 constexpr SubsetTable make_subset_table() {
     SubsetTable t{};
-    int k = 0;
-    for (int size = 1; size <= 7; ++size) {
-        t.start[size] = (uint8_t)k;
-        for (int S = 1; S < 128; ++S) {
-            int c = 0;
-            for (int b = 0; b < 7; ++b) c += (S >> b) & 1;
-            if (c == size) t.set[k++] = (uint8_t)S;
+    const int first_row[8] = {0, 0, 0, 1, 3, 5, 6, 0};
+    int count[8] = {};
+    for (int S = 1; S < 128; ++S) {
+        int size = 0;
+        for (int b = 0; b < 7; ++b) size += (S >> b) & 1;
+        if (size < 2 || size > 6) continue;
+        const int k = count[size]++;
+        if (size == 6) {
+            for (int q = 0; q < 4; ++q) t.set[6][4 * k + q] = (uint8_t)S;
+        } else {
+            t.set[first_row[size] + k / 32][k % 32] = (uint8_t)S;
         }
     }
-    t.start[0] = 0;
-    t.start[8] = (uint8_t)k;
     return t;
 }
-__constant__ SubsetTable c_subsets = make_subset_table();
+__device__ const SubsetTable d_subsets = make_subset_table();
 
-struct TreeletSmem {
-    float llo[kTreeletLeaves][3], lhi[kTreeletLeaves][3];
-    int32_t lcnt[kTreeletLeaves], leaf[kTreeletLeaves], inner[kTreeletLeaves - 1];
-    float cost[1 << kTreeletLeaves];
-    float slo[1 << kTreeletLeaves][3], shi[1 << kTreeletLeaves][3];  // subset boxes
-    uint8_t part[1 << kTreeletLeaves];
+// A lane's subsets: of 2, 3 (two), 4 (two), 5 and 6 leaves; 0 where it has none.
+struct LaneSubsets {
+    int s2, s3[2], s4[2], s5, s6;
 };
 
-// The i-th partition {P, S ^ P} of S in restructure()'s order: P holds the
-// lowest leaf of S, and P runs down from S - 1 over the subsets of S.
-__device__ inline int nth_partition(int S, int i) {
-    const int low = S & -S;
-    const int R = S ^ low;  // the other leaves
-    // Q = the i-th largest proper subset of R: the bits of (2^|R| - 2 - i)
-    // deposited into the positions of R.
-    const int nb = __popc(R);
-    int v = (1 << nb) - 2 - i, Q = 0, r = R;
-    for (int b = 0; b < nb; ++b) {
-        const int bit = r & -r;
-        if (v & (1 << b)) Q |= bit;
-        r ^= bit;
-    }
-    return low | Q;
+// The bits of v deposited into the set bits of R.
+__device__ inline int deposit(int v, int R) {
+    int Q = 0;
+    for (int r = R, b = 0; r; r &= r - 1, ++b)
+        if (v & (1 << b)) Q |= r & -r;
+    return Q;
 }
 
-// The box of subset S (two or more leaves) from the box of S without its
-// highest leaf, already in the table, and that leaf's box; min / max are
-// exact in any order, so it equals restructure()'s box of the same leaves.
-__device__ void subset_box_s(TreeletSmem& t, int S, float lo[3], float hi[3]) {
-    const int high = 31 - __clz(S);
-    const int R = S & ~(1 << high);
-    for (int a = 0; a < 3; ++a) {
-        lo[a] = fminf(t.slo[R][a], t.llo[high][a]);
-        hi[a] = fmaxf(t.shi[R][a], t.lhi[high][a]);
-        t.slo[S][a] = lo[a];
-        t.shi[S][a] = hi[a];
+__device__ inline float subset_area(const TreeletSmem& t, int S) {
+    float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
+    for (int r = S; r; r &= r - 1) {
+        const int q = __ffs(r) - 1;
+        const float4 l = t.lo[q], h = t.hi[q];
+        lo[0] = fminf(lo[0], l.x); lo[1] = fminf(lo[1], l.y); lo[2] = fminf(lo[2], l.z);
+        hi[0] = fmaxf(hi[0], h.x); hi[1] = fmaxf(hi[1], h.y); hi[2] = fmaxf(hi[2], h.z);
     }
+    return half_area(lo, hi);
+}
+
+// The first minimum of a subset's partitions from Q (the part of P besides
+// the lowest leaf) down through `count` of them.
+__device__ inline void best_partition(const TreeletSmem& t, int S, int Q, int count, float& bc, int& bp) {
+    const int low = S & -S, R = S ^ low;
+    bc = FLT_MAX;
+    bp = 0;
+#pragma unroll 4
+    for (int i = 0; i < count; ++i) {
+        const int P = low | Q;
+        const float c = __fadd_rn(t.cost[P], t.cost[S ^ P]);
+        if (c < bc) { bc = c; bp = P; }
+        Q = (Q - 1) & R;
+    }
+}
+
+__device__ inline void cost_subset(TreeletSmem& t, int S, int size) {
+    if (S == 0) return;
+    const int R = S & (S - 1);
+    float bc;
+    int bp;
+    best_partition(t, S, (R - 1) & R, (1 << (size - 1)) - 1, bc, bp);
+    t.cost[S] = __fadd_rn(__fmul_rn(kCt, subset_area(t, S)), bc);
+    t.part[S] = (uint8_t)bp;
 }
 
 // The whole warp restructures the treelet rooted at `root` (warp-uniform).
 __device__ void restructure_warp(BNode* nodes, const NodeBox* leaves, int32_t* leaf_parent, int32_t root,
-                                 float root_cost, TreeletSmem& t) {
+                                 float root_cost, TreeletSmem& t, const LaneSubsets& mine) {
     const unsigned lane = threadIdx.x & 31u;
     // Grow the treelet: lane q holds leaf q.
     int32_t my_leaf = -1;
-    NodeBox mine{};
-    float marea = -1.f;
-    int n_in = 1, n_leaf = 2;
-    if (lane < 2) {
-        my_leaf = lane == 0 ? ld_left(nodes, root) : ld_right(nodes, root);
-        mine = child_box(nodes, leaves, my_leaf);
-        marea = half_area(mine.lo, mine.hi);
-    }
-    if (lane == 0) t.inner[0] = root;
+    int2 links = make_int2(0, 0);
+    NodeBox box{};
+    unsigned key = 0u;  // orders the leaves that are nodes by area
+    auto take = [&](int32_t code) {
+        my_leaf = code;
+        if (code >= 0) links = __ldcg(reinterpret_cast<const int2*>(&nodes[code].left));
+        box = child_box(nodes, leaves, code);
+        const float area = half_area(box.lo, box.hi);
+        key = code >= 0 && area > -1.f ? (__float_as_uint(area) & 0x7FFFFFFFu) + 1u : 0u;
+    };
+    const int2 top = __ldcg(reinterpret_cast<const int2*>(&nodes[root].left));
+    if (lane < 2) take(lane == 0 ? top.x : top.y);
+    int n_leaf = 2;
+    int my_inner = root;  // lane q: the q-th node of the treelet
     while (n_leaf < kTreeletLeaves) {
         // the first leaf of the largest area that is a node (restructure()'s scan)
-        float a = ((int)lane < n_leaf && my_leaf >= 0) ? marea : -1.f;
-        int best = ((int)lane < n_leaf && my_leaf >= 0) ? (int)lane : 64;
-        for (int o = 16; o > 0; o >>= 1) {
-            const float a2 = __shfl_xor_sync(kWarpAll, a, o);
-            const int b2 = __shfl_xor_sync(kWarpAll, best, o);
-            if (a2 > a || (a2 == a && b2 < best)) { a = a2; best = b2; }
-        }
-        if (best >= 64 || !(a > -1.f)) break;
+        const unsigned most = __reduce_max_sync(kWarpAll, key);
+        if (most == 0u) break;
+        const int best = __ffs(__ballot_sync(kWarpAll, key == most)) - 1;
         const int32_t x = __shfl_sync(kWarpAll, my_leaf, best);
-        if (lane == 0) t.inner[n_in] = x;
-        ++n_in;
-        if ((int)lane == best || (int)lane == n_leaf) {
-            my_leaf = (int)lane == best ? ld_left(nodes, x) : ld_right(nodes, x);
-            mine = child_box(nodes, leaves, my_leaf);
-            marea = half_area(mine.lo, mine.hi);
-        }
+        const int32_t l = __shfl_sync(kWarpAll, links.x, best), r = __shfl_sync(kWarpAll, links.y, best);
+        if ((int)lane == n_leaf - 1) my_inner = x;
+        if ((int)lane == best || (int)lane == n_leaf) take((int)lane == best ? l : r);
         ++n_leaf;
     }
     if (n_leaf < 3) return;
     if ((int)lane < n_leaf) {
-        for (int a = 0; a < 3; ++a) {
-            t.llo[lane][a] = mine.lo[a];
-            t.lhi[lane][a] = mine.hi[a];
-            t.slo[1 << lane][a] = mine.lo[a];
-            t.shi[1 << lane][a] = mine.hi[a];
-        }
-        t.lcnt[lane] = mine.count;
+        t.lo[lane] = make_float4(box.lo[0], box.lo[1], box.lo[2], 0.f);
+        t.hi[lane] = make_float4(box.hi[0], box.hi[1], box.hi[2], 0.f);
+        t.count[lane] = box.count;
         t.leaf[lane] = my_leaf;
-        t.cost[1 << lane] = mine.cost;
-        t.part[1 << lane] = 0;
+        t.inner[lane] = my_inner;
+        t.cost[1 << lane] = box.cost;
     }
     __syncwarp();
     const int full = (1 << n_leaf) - 1;
-    for (int size = 2; size <= n_leaf; ++size) {
-        const int first = c_subsets.start[size], end = c_subsets.start[size + 1];
-        if (size < 7) {
-            // one subset per lane
-            for (int e = first + (int)lane; e < end; e += 32) {
-                const int S = c_subsets.set[e];
-                if (S > full) continue;
-                float slo[3], shi[3];
-                subset_box_s(t, S, slo, shi);
-                const int low = __ffs(S) - 1;
-                float bc = FLT_MAX;
-                int bp = 0;
-                for (int P = (S - 1) & S; P > 0; P = (P - 1) & S) {
-                    if (!(P & (1 << low))) continue;
-                    const float c = __fadd_rn(t.cost[P], t.cost[S ^ P]);
-                    if (c < bc) { bc = c; bp = P; }
-                }
-                t.cost[S] = __fadd_rn(__fmul_rn(kCt, half_area(slo, shi)), bc);
-                t.part[S] = (uint8_t)bp;
-            }
-        } else {
-            // one subset at a time, its partitions over the lanes
-            for (int e = first; e < end; ++e) {
-                const int S = c_subsets.set[e];
-                if (S > full) continue;
-                const int n_part = (1 << (__popc(S) - 1)) - 1;
-                float bc = FLT_MAX;
-                int bi = 1 << 30;
-                for (int i = (int)lane; i < n_part; i += 32) {
-                    const int P = nth_partition(S, i);
-                    const float c = __fadd_rn(t.cost[P], t.cost[S ^ P]);
-                    if (c < bc) { bc = c; bi = i; }
-                }
-                for (int o = 16; o > 0; o >>= 1) {
-                    const float c2 = __shfl_xor_sync(kWarpAll, bc, o);
-                    const int i2 = __shfl_xor_sync(kWarpAll, bi, o);
-                    if (c2 < bc || (c2 == bc && i2 < bi)) { bc = c2; bi = i2; }
-                }
-                if (lane == 0) {
-                    float slo[3], shi[3];
-                    subset_box_s(t, S, slo, shi);
-                    t.cost[S] = __fadd_rn(__fmul_rn(kCt, half_area(slo, shi)), bc);
-                    t.part[S] = (uint8_t)(bi < n_part ? nth_partition(S, bi) : 0);
-                }
-                __syncwarp();
-            }
+    auto in = [&](int S) { return S <= full ? S : 0; };
+    cost_subset(t, in(mine.s2), 2);
+    __syncwarp();
+    cost_subset(t, in(mine.s3[0]), 3);
+    cost_subset(t, in(mine.s3[1]), 3);
+    __syncwarp();
+    cost_subset(t, in(mine.s4[0]), 4);
+    cost_subset(t, in(mine.s4[1]), 4);
+    __syncwarp();
+    cost_subset(t, in(mine.s5), 5);
+    __syncwarp();
+    {
+        // 6 leaves: 31 partitions over four lanes, eight each in order
+        const int S = in(mine.s6), R = S & (S - 1), chunk = (int)(lane & 3u);
+        float bc = FLT_MAX;
+        int bp = 0, at = chunk;
+        if (S) best_partition(t, S, deposit(30 - 8 * chunk, R), chunk == 3 ? 7 : 8, bc, bp);
+        for (int o = 2; o > 0; o >>= 1) {
+            const float c2 = __shfl_xor_sync(kWarpAll, bc, o);
+            const int p2 = __shfl_xor_sync(kWarpAll, bp, o), a2 = __shfl_xor_sync(kWarpAll, at, o);
+            if (c2 < bc || (c2 == bc && a2 < at)) { bc = c2; bp = p2; at = a2; }
+        }
+        if (S && chunk == 0) {
+            t.cost[S] = __fadd_rn(__fmul_rn(kCt, subset_area(t, S)), bc);
+            t.part[S] = (uint8_t)bp;
+        }
+    }
+    __syncwarp();
+    float new_cost;
+    if (n_leaf == kTreeletLeaves) {
+        // 7 leaves: 63 partitions, two per lane
+        const int S = full, R = S ^ 1;
+        float bc = FLT_MAX;
+        int bp = 0, at = 64;
+        for (int i = (int)lane; i < 63; i += 32) {
+            const int P = 1 | (((62 - i) << 1) & R);  // R's bits are 1..6: the deposit is a shift
+            const float c = __fadd_rn(t.cost[P], t.cost[S ^ P]);
+            if (c < bc) { bc = c; bp = P; at = i; }
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            const float c2 = __shfl_xor_sync(kWarpAll, bc, o);
+            const int p2 = __shfl_xor_sync(kWarpAll, bp, o), a2 = __shfl_xor_sync(kWarpAll, at, o);
+            if (c2 < bc || (c2 == bc && a2 < at)) { bc = c2; bp = p2; at = a2; }
+        }
+        new_cost = __fadd_rn(__fmul_rn(kCt, subset_area(t, S)), bc);
+        if (lane == 0) {
+            t.cost[S] = new_cost;
+            t.part[S] = (uint8_t)bp;
         }
         __syncwarp();
+    } else {
+        new_cost = t.cost[full];
     }
-    if (lane == 0 && t.cost[full] < 0.999f * root_cost) {
-        // every subset the new tree splits must have a split (finite costs);
-        // check before writing anything
-        bool ok = true;
-        {
-            int st[kTreeletLeaves], sp = 0;
-            st[sp++] = full;
-            while (sp > 0 && ok) {
-                const int S = st[--sp];
-                const int P = t.part[S];
-                if (P == 0 || (P & ~S) != 0 || P == S) { ok = false; break; }
-                if (P & (P - 1)) st[sp++] = P;
-                if ((S ^ P) & ((S ^ P) - 1)) st[sp++] = S ^ P;
-                if (sp > kTreeletLeaves - 1) ok = false;
+    if (!(new_cost < 0.999f * root_cost)) return;
+    // The new treelet, breadth first: node k has leaf set set[k] and becomes
+    // inner[k].  Every set it splits must have a split (finite costs); checked
+    // before anything is written.
+    bool ok = true;
+    if (lane == 0) {
+        int n = 1;
+        t.set[0] = full;
+        for (int q = 0; q < n && ok; ++q) {
+            const int S = t.set[q], P = t.part[S];
+            if (P == 0 || (P & ~S) != 0 || P == S) { ok = false; break; }
+            for (int side = 0; side < 2; ++side) {
+                const int T = side ? S ^ P : P;
+                if ((T & (T - 1)) == 0) continue;
+                if (n >= n_leaf - 1) { ok = false; break; }
+                t.set[n++] = T;
             }
         }
-        if (ok) {
-            // rebuild top-down: subset -> node, internal nodes taken from `inner`
-            int32_t st_set[kTreeletLeaves], st_node[kTreeletLeaves];
-            int sp = 0, used = 1;
-            st_set[sp] = full;
-            st_node[sp++] = root;
-            while (sp > 0) {
-                --sp;
-                const int S = st_set[sp];
-                const int32_t nd = st_node[sp];
-                const int P = t.part[S];
-                const int side[2] = {P, S ^ P};
-                int32_t code[2];
-                for (int c = 0; c < 2; ++c) {
-                    const int T = side[c];
-                    if ((T & (T - 1)) == 0) {
-                        code[c] = t.leaf[__ffs(T) - 1];
-                        if (code[c] >= 0) nodes[code[c]].parent = nd;
-                        else leaf_parent[~code[c]] = nd;
-                    } else {
-                        const int32_t ni = t.inner[used++];
-                        code[c] = ni;
-                        nodes[ni].parent = nd;
-                        st_set[sp] = T;
-                        st_node[sp++] = ni;
-                    }
-                }
-                BNode& b = nodes[nd];
-                b.left = code[0];
-                b.right = code[1];
-                NodeBox nb;
-                for (int a = 0; a < 3; ++a) { nb.lo[a] = t.slo[S][a]; nb.hi[a] = t.shi[S][a]; }
-                nb.count = 0;
-                for (int q = 0; q < n_leaf; ++q)
-                    if (S & (1 << q)) nb.count += t.lcnt[q];
-                nb.cost = t.cost[S];
-                store_box(&b.b, nb);
+        ok = ok && n == n_leaf - 1;
+    }
+    if (!__shfl_sync(kWarpAll, (int)ok, 0)) return;
+    __syncwarp();
+    if ((int)lane < n_leaf - 1) {
+        const int S = t.set[lane], P = t.part[S];
+        const int32_t nd = t.inner[lane];
+        int32_t code[2];
+        for (int side = 0; side < 2; ++side) {
+            const int T = side ? S ^ P : P;
+            if ((T & (T - 1)) == 0) {
+                code[side] = t.leaf[__ffs(T) - 1];
+                if (code[side] >= 0) nodes[code[side]].parent = nd;
+                else leaf_parent[~code[side]] = nd;
+            } else {
+                int q = (int)lane + 1;
+                while (q < n_leaf - 2 && t.set[q] != T) ++q;
+                code[side] = t.inner[q];
+                nodes[t.inner[q]].parent = nd;
             }
-            __threadfence();
         }
+        *reinterpret_cast<int2*>(&nodes[nd].left) = make_int2(code[0], code[1]);
+        NodeBox nb;
+        for (int a = 0; a < 3; ++a) { nb.lo[a] = FLT_MAX; nb.hi[a] = -FLT_MAX; }
+        nb.count = 0;
+        for (int r = S; r; r &= r - 1) {
+            const int q = __ffs(r) - 1;
+            const float4 l = t.lo[q], h = t.hi[q];
+            nb.lo[0] = fminf(nb.lo[0], l.x); nb.lo[1] = fminf(nb.lo[1], l.y); nb.lo[2] = fminf(nb.lo[2], l.z);
+            nb.hi[0] = fmaxf(nb.hi[0], h.x); nb.hi[1] = fmaxf(nb.hi[1], h.y); nb.hi[2] = fmaxf(nb.hi[2], h.z);
+            nb.count += t.count[q];
+        }
+        nb.cost = t.cost[S];
+        store_box(&nodes[nd].b, nb);
+        __threadfence();
     }
     __syncwarp();
 }
@@ -890,6 +914,14 @@ __global__ void __launch_bounds__(kTreeletWarpBlock) treelet_warp_kernel(
     TreeletSmem& t = smem[threadIdx.x / 32];
     const unsigned lane = threadIdx.x & 31u;
     const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    LaneSubsets mine;
+    mine.s2 = d_subsets.set[0][lane];
+    mine.s3[0] = d_subsets.set[1][lane];
+    mine.s3[1] = d_subsets.set[2][lane];
+    mine.s4[0] = d_subsets.set[3][lane];
+    mine.s4[1] = d_subsets.set[4][lane];
+    mine.s5 = d_subsets.set[5][lane];
+    mine.s6 = d_subsets.set[6][lane];
     int32_t node = p < n ? leaf_parent[p] : -1;
     for (;;) {
         bool go = node >= 0;
@@ -914,7 +946,7 @@ __global__ void __launch_bounds__(kTreeletWarpBlock) treelet_warp_kernel(
             want &= want - 1;
             const int32_t root = __shfl_sync(kWarpAll, node, src);
             const float rc = __shfl_sync(kWarpAll, cost, src);
-            restructure_warp(nodes, leaves, leaf_parent, root, rc, t);
+            restructure_warp(nodes, leaves, leaf_parent, root, rc, t, mine);
         }
         if (go) node = ld_parent(nodes, node);
         if (__ballot_sync(kWarpAll, node >= 0) == 0u) break;

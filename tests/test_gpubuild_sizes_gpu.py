@@ -16,7 +16,7 @@ pytestmark = pytest.mark.gpu
 def test_build_sizes(rq, po, n, method):
     import torch
     from cwbvh_b200 import workloads as W
-    V, I = W.scene_of_size(n, n + 40)
+    V, I = W.scene_of_size(n, n + n // 8 + 100)
     assert I.shape[0] >= n
     I = np.ascontiguousarray(np.random.default_rng(n).permutation(I)[:n])
     v, i = torch.from_numpy(V).cuda(), torch.from_numpy(I).cuda()
