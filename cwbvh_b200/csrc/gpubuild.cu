@@ -669,7 +669,7 @@ __global__ void treelet_kernel(int64_t n, const NodeBox* leaves, BNode* nodes, i
 // table in constant memory costs a pass per lane), only partitions that hold
 // the lowest leaf are formed, and a subset's box is made from its leaves'
 // (two 16-byte reads each) so that the table is 1 KB and not 4 per warp.  Two
-// passes over 500,000 triangles: 2,854 -> TREELET_US us.
+// passes over 500,000 triangles: 2,854 -> 1,636 us.
 constexpr unsigned kWarpAll = 0xFFFFFFFFu;
 
 struct TreeletSmem {
