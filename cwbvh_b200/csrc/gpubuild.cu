@@ -718,10 +718,12 @@ __device__ inline int deposit(int v, int R) {
     return Q;
 }
 
+template <int SIZE>
 __device__ inline float subset_area(const TreeletSmem& t, int S) {
     float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-    for (int r = S; r; r &= r - 1) {
-        const int q = __ffs(r) - 1;
+#pragma unroll
+    for (int i = 0; i < SIZE; ++i, S &= S - 1) {
+        const int q = __ffs(S) - 1;
         const float4 l = t.lo[q], h = t.hi[q];
         lo[0] = fminf(lo[0], l.x); lo[1] = fminf(lo[1], l.y); lo[2] = fminf(lo[2], l.z);
         hi[0] = fmaxf(hi[0], h.x); hi[1] = fmaxf(hi[1], h.y); hi[2] = fmaxf(hi[2], h.z);
@@ -729,49 +731,68 @@ __device__ inline float subset_area(const TreeletSmem& t, int S) {
     return half_area(lo, hi);
 }
 
-// The first minimum of a subset's partitions from Q (the part of P besides
-// the lowest leaf) down through `count` of them.
-__device__ inline void best_partition(const TreeletSmem& t, int S, int Q, int count, float& bc, int& bp) {
+// The first minimum of COUNT of a subset's partitions, from Q (the part of P
+// besides the lowest leaf) down; the last `skip` of them do not count.
+template <int COUNT>
+__device__ inline void best_partition(const TreeletSmem& t, int S, int Q, int skip, float& bc, int& bp) {
     const int low = S & -S, R = S ^ low;
     bc = FLT_MAX;
     bp = 0;
 #pragma unroll 4
-    for (int i = 0; i < count; ++i) {
+    for (int i = 0; i < COUNT; ++i) {
         const int P = low | Q;
         const float c = __fadd_rn(t.cost[P], t.cost[S ^ P]);
-        if (c < bc) { bc = c; bp = P; }
+        if (c < bc && i < COUNT - skip) { bc = c; bp = P; }
         Q = (Q - 1) & R;
     }
 }
 
-__device__ inline void cost_subset(TreeletSmem& t, int S, int size) {
+template <int SIZE>
+__device__ inline void cost_subset(TreeletSmem& t, int S) {
     if (S == 0) return;
     const int R = S & (S - 1);
     float bc;
     int bp;
-    best_partition(t, S, (R - 1) & R, (1 << (size - 1)) - 1, bc, bp);
-    t.cost[S] = __fadd_rn(__fmul_rn(kCt, subset_area(t, S)), bc);
+    best_partition<(1 << (SIZE - 1)) - 1>(t, S, (R - 1) & R, 0, bc, bp);
+    t.cost[S] = __fadd_rn(__fmul_rn(kCt, subset_area<SIZE>(t, S)), bc);
     t.part[S] = (uint8_t)bp;
 }
 
-// The whole warp restructures the treelet rooted at `root` (warp-uniform).
+// The whole warp restructures the treelet rooted at `root` (warp-uniform),
+// which lane `src` has read: its children and their boxes.
 __device__ void restructure_warp(BNode* nodes, const NodeBox* leaves, int32_t* leaf_parent, int32_t root,
-                                 float root_cost, TreeletSmem& t, const LaneSubsets& mine) {
+                                 float root_cost, int src, const int2& src_links, const NodeBox& src_left,
+                                 const NodeBox& src_right, TreeletSmem& t, const LaneSubsets& mine) {
     const unsigned lane = threadIdx.x & 31u;
     // Grow the treelet: lane q holds leaf q.
     int32_t my_leaf = -1;
     int2 links = make_int2(0, 0);
     NodeBox box{};
     unsigned key = 0u;  // orders the leaves that are nodes by area
-    auto take = [&](int32_t code) {
+    auto take = [&](int32_t code, const NodeBox* known) {
         my_leaf = code;
         if (code >= 0) links = __ldcg(reinterpret_cast<const int2*>(&nodes[code].left));
-        box = child_box(nodes, leaves, code);
+        if (known) box = *known;
+        else box = child_box(nodes, leaves, code);
         const float area = half_area(box.lo, box.hi);
         key = code >= 0 && area > -1.f ? (__float_as_uint(area) & 0x7FFFFFFFu) + 1u : 0u;
     };
-    const int2 top = __ldcg(reinterpret_cast<const int2*>(&nodes[root].left));
-    if (lane < 2) take(lane == 0 ? top.x : top.y);
+    {
+        NodeBox l, r;
+        for (int a = 0; a < 3; ++a) {
+            l.lo[a] = __shfl_sync(kWarpAll, src_left.lo[a], src);
+            l.hi[a] = __shfl_sync(kWarpAll, src_left.hi[a], src);
+            r.lo[a] = __shfl_sync(kWarpAll, src_right.lo[a], src);
+            r.hi[a] = __shfl_sync(kWarpAll, src_right.hi[a], src);
+        }
+        l.cost = __shfl_sync(kWarpAll, src_left.cost, src);
+        l.count = __shfl_sync(kWarpAll, src_left.count, src);
+        r.cost = __shfl_sync(kWarpAll, src_right.cost, src);
+        r.count = __shfl_sync(kWarpAll, src_right.count, src);
+        const int32_t lc = __shfl_sync(kWarpAll, src_links.x, src), rc = __shfl_sync(kWarpAll, src_links.y, src);
+        if (lane == 1) l = r;
+        if (lane < 2) take(lane == 0 ? lc : rc, &l);
+    }
     int n_leaf = 2;
     int my_inner = root;  // lane q: the q-th node of the treelet
     while (n_leaf < kTreeletLeaves) {
@@ -782,7 +803,7 @@ __device__ void restructure_warp(BNode* nodes, const NodeBox* leaves, int32_t* l
         const int32_t x = __shfl_sync(kWarpAll, my_leaf, best);
         const int32_t l = __shfl_sync(kWarpAll, links.x, best), r = __shfl_sync(kWarpAll, links.y, best);
         if ((int)lane == n_leaf - 1) my_inner = x;
-        if ((int)lane == best || (int)lane == n_leaf) take((int)lane == best ? l : r);
+        if ((int)lane == best || (int)lane == n_leaf) take((int)lane == best ? l : r, nullptr);
         ++n_leaf;
     }
     if (n_leaf < 3) return;
@@ -797,29 +818,29 @@ __device__ void restructure_warp(BNode* nodes, const NodeBox* leaves, int32_t* l
     __syncwarp();
     const int full = (1 << n_leaf) - 1;
     auto in = [&](int S) { return S <= full ? S : 0; };
-    cost_subset(t, in(mine.s2), 2);
+    cost_subset<2>(t, in(mine.s2));
     __syncwarp();
-    cost_subset(t, in(mine.s3[0]), 3);
-    cost_subset(t, in(mine.s3[1]), 3);
+    cost_subset<3>(t, in(mine.s3[0]));
+    cost_subset<3>(t, in(mine.s3[1]));
     __syncwarp();
-    cost_subset(t, in(mine.s4[0]), 4);
-    cost_subset(t, in(mine.s4[1]), 4);
+    cost_subset<4>(t, in(mine.s4[0]));
+    cost_subset<4>(t, in(mine.s4[1]));
     __syncwarp();
-    cost_subset(t, in(mine.s5), 5);
+    cost_subset<5>(t, in(mine.s5));
     __syncwarp();
     {
         // 6 leaves: 31 partitions over four lanes, eight each in order
         const int S = in(mine.s6), R = S & (S - 1), chunk = (int)(lane & 3u);
         float bc = FLT_MAX;
         int bp = 0, at = chunk;
-        if (S) best_partition(t, S, deposit(30 - 8 * chunk, R), chunk == 3 ? 7 : 8, bc, bp);
+        if (S) best_partition<8>(t, S, deposit(30 - 8 * chunk, R), chunk == 3 ? 1 : 0, bc, bp);
         for (int o = 2; o > 0; o >>= 1) {
             const float c2 = __shfl_xor_sync(kWarpAll, bc, o);
             const int p2 = __shfl_xor_sync(kWarpAll, bp, o), a2 = __shfl_xor_sync(kWarpAll, at, o);
             if (c2 < bc || (c2 == bc && a2 < at)) { bc = c2; bp = p2; at = a2; }
         }
         if (S && chunk == 0) {
-            t.cost[S] = __fadd_rn(__fmul_rn(kCt, subset_area(t, S)), bc);
+            t.cost[S] = __fadd_rn(__fmul_rn(kCt, subset_area<6>(t, S)), bc);
             t.part[S] = (uint8_t)bp;
         }
     }
@@ -840,7 +861,7 @@ __device__ void restructure_warp(BNode* nodes, const NodeBox* leaves, int32_t* l
             const int p2 = __shfl_xor_sync(kWarpAll, bp, o), a2 = __shfl_xor_sync(kWarpAll, at, o);
             if (c2 < bc || (c2 == bc && a2 < at)) { bc = c2; bp = p2; at = a2; }
         }
-        new_cost = __fadd_rn(__fmul_rn(kCt, subset_area(t, S)), bc);
+        new_cost = __fadd_rn(__fmul_rn(kCt, subset_area<7>(t, S)), bc);
         if (lane == 0) {
             t.cost[S] = new_cost;
             t.part[S] = (uint8_t)bp;
@@ -908,7 +929,7 @@ __device__ void restructure_warp(BNode* nodes, const NodeBox* leaves, int32_t* l
 
 constexpr int kTreeletWarpBlock = 128;
 
-__global__ void __launch_bounds__(kTreeletWarpBlock) treelet_warp_kernel(
+__global__ void __launch_bounds__(kTreeletWarpBlock, 8) treelet_warp_kernel(
         int64_t n, const NodeBox* leaves, BNode* nodes, int32_t* leaf_parent, int32_t* arrivals, int min_count) {
     __shared__ TreeletSmem smem[kTreeletWarpBlock / 32];
     TreeletSmem& t = smem[threadIdx.x / 32];
@@ -933,9 +954,16 @@ __global__ void __launch_bounds__(kTreeletWarpBlock) treelet_warp_kernel(
         if (!go) node = -1;
         float cost = 0.f;
         bool due = false;
+        int32_t parent = -1;  // read ahead of the treelet: only treelets further up change it
+        int2 links = make_int2(0, 0);
+        NodeBox left{}, right{};
         if (go) {
-            const NodeBox b = join(child_box(nodes, leaves, ld_left(nodes, node)),
-                                   child_box(nodes, leaves, ld_right(nodes, node)));
+            const int4 nd = __ldcg(reinterpret_cast<const int4*>(&nodes[node]));
+            links = make_int2(nd.x, nd.y);
+            parent = nd.z;
+            left = child_box(nodes, leaves, links.x);
+            right = child_box(nodes, leaves, links.y);
+            const NodeBox b = join(left, right);
             cost = b.cost;
             __stcg(&nodes[node].b.cost, cost);
             due = b.count >= min_count;
@@ -946,9 +974,9 @@ __global__ void __launch_bounds__(kTreeletWarpBlock) treelet_warp_kernel(
             want &= want - 1;
             const int32_t root = __shfl_sync(kWarpAll, node, src);
             const float rc = __shfl_sync(kWarpAll, cost, src);
-            restructure_warp(nodes, leaves, leaf_parent, root, rc, t, mine);
+            restructure_warp(nodes, leaves, leaf_parent, root, rc, src, links, left, right, t, mine);
         }
-        if (go) node = ld_parent(nodes, node);
+        if (go) node = parent;
         if (__ballot_sync(kWarpAll, node >= 0) == 0u) break;
     }
 }
