@@ -57,7 +57,8 @@ struct __align__(16) NodeBox {
 struct __align__(16) BNode {
     int32_t left, right;  // >= 0: internal node, < 0: leaf ~(sorted position)
     int32_t parent;       // -1 at the root
-    int32_t pad;
+    uint32_t stamps;      // treelet passes (from 1): low half the last that rewrote this node, high half the
+                          // last that rewrote this node or one below it on its way up
     NodeBox b;
 };
 static_assert(sizeof(NodeBox) == 32 && sizeof(BNode) == 48, "node layout");
@@ -422,6 +423,7 @@ __global__ void radix_tree_kernel(const uint64_t* k, int64_t n, BNode* nodes, in
     if (nd.right >= 0) nodes[nd.right].parent = (int32_t)i;
     else leaf_parent[gamma + 1] = (int32_t)i;
     if (i == 0) nd.parent = -1;
+    nd.stamps = 0u;
 }
 
 // The triangle of a sorted key: its low idx_bits bits (idx_mask).
@@ -664,6 +666,14 @@ __global__ void treelet_kernel(int64_t n, const NodeBox* leaves, BNode* nodes, i
 // partition is the first minimum in its order there, so the trees are
 // identical.
 //
+// From the second pass on a treelet is due only if its subtree is not the one
+// that the pass before left its root with: that pass rewrote the root (by its
+// own treelet or as an inner node of one further up, which any change further
+// down that the root did not see also does), or this pass rewrote a node below.
+// Another treelet would find what it found before: the same trees.  Second pass
+// over 2M triangles (spheres) 1,930 -> 1,175 us, 280,000 (city) 440 -> 370 us;
+// nothing where the first pass rewrote nearly all (heightfield 690 -> 670 us).
+//
 // Bound by the warp's own chain of steps and, up the tree, by the chain of
 // treelets.  A lane's subsets are worked out once and kept in registers (a
 // table in constant memory costs a pass per lane), only partitions that hold
@@ -761,7 +771,7 @@ __device__ inline void cost_subset(TreeletSmem& t, int S) {
 // The whole warp restructures the treelet rooted at `root` (warp-uniform),
 // which lane `src` has read: its children and their boxes.
 __device__ void restructure_warp(BNode* nodes, const NodeBox* leaves, int32_t* leaf_parent, int32_t root,
-                                 float root_cost, int src, const int2& src_links, const NodeBox& src_left,
+                                 float root_cost, unsigned stamps, int src, const int2& src_links, const NodeBox& src_left,
                                  const NodeBox& src_right, TreeletSmem& t, const LaneSubsets& mine) {
     const unsigned lane = threadIdx.x & 31u;
     // Grow the treelet: lane q holds leaf q.
@@ -910,6 +920,7 @@ __device__ void restructure_warp(BNode* nodes, const NodeBox* leaves, int32_t* l
             }
         }
         *reinterpret_cast<int2*>(&nodes[nd].left) = make_int2(code[0], code[1]);
+        nodes[nd].stamps = stamps;
         NodeBox nb;
         for (int a = 0; a < 3; ++a) { nb.lo[a] = FLT_MAX; nb.hi[a] = -FLT_MAX; }
         nb.count = 0;
@@ -930,7 +941,8 @@ __device__ void restructure_warp(BNode* nodes, const NodeBox* leaves, int32_t* l
 constexpr int kTreeletWarpBlock = 128;
 
 __global__ void __launch_bounds__(kTreeletWarpBlock, 8) treelet_warp_kernel(
-        int64_t n, const NodeBox* leaves, BNode* nodes, int32_t* leaf_parent, int32_t* arrivals, int min_count) {
+        int64_t n, const NodeBox* leaves, BNode* nodes, int32_t* leaf_parent, int32_t* arrivals, int min_count,
+        unsigned pass) {
     __shared__ TreeletSmem smem[kTreeletWarpBlock / 32];
     TreeletSmem& t = smem[threadIdx.x / 32];
     const unsigned lane = threadIdx.x & 31u;
@@ -966,7 +978,12 @@ __global__ void __launch_bounds__(kTreeletWarpBlock, 8) treelet_warp_kernel(
             const NodeBox b = join(left, right);
             cost = b.cost;
             __stcg(&nodes[node].b.cost, cost);
-            due = b.count >= min_count;
+            const bool below = (links.x >= 0 && __ldcg(&nodes[links.x].stamps) >> 16 == pass) ||
+                               (links.y >= 0 && __ldcg(&nodes[links.y].stamps) >> 16 == pass);
+            const unsigned own = (unsigned)nd.w & 0xFFFFu;
+            due = b.count >= min_count && (pass == 1u || own == pass - 1u || below);
+            // a treelet that is rewritten stamps its nodes itself
+            if (below) __stcg(&nodes[node].stamps, own | (pass << 16));
         }
         unsigned want = __ballot_sync(kWarpAll, due);
         while (want) {
@@ -974,7 +991,7 @@ __global__ void __launch_bounds__(kTreeletWarpBlock, 8) treelet_warp_kernel(
             want &= want - 1;
             const int32_t root = __shfl_sync(kWarpAll, node, src);
             const float rc = __shfl_sync(kWarpAll, cost, src);
-            restructure_warp(nodes, leaves, leaf_parent, root, rc, src, links, left, right, t, mine);
+            restructure_warp(nodes, leaves, leaf_parent, root, rc, pass | (pass << 16), src, links, left, right, t, mine);
         }
         if (go) node = parent;
         if (__ballot_sync(kWarpAll, node >= 0) == 0u) break;
@@ -2019,7 +2036,8 @@ static rq_status build_scene(const float* vertices, int64_t nv, const int32_t* i
                 treelet_kernel<<<blocks_of(n, 128), 128, 0, s>>>(n, leaves, bn, leaf_parent, arrivals, kTreeletLeaves);
             else
                 treelet_warp_kernel<<<blocks_of(n, kTreeletWarpBlock), kTreeletWarpBlock, 0, s>>>(
-                    n, leaves, bn, leaf_parent, arrivals, kTreeletLeaves);
+                    n, leaves, bn, leaf_parent, arrivals, kTreeletLeaves,
+                    pass < 65535 ? (unsigned)pass + 1u : 1u);  // pass 1 takes every treelet; stamps have 16 bits
             ok(cudaGetLastError(), "rq_build_scene_gpu");
         }
         if (st == RQ_OK) {
