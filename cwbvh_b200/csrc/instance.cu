@@ -73,8 +73,18 @@ __device__ __forceinline__ void cwbvh_visit(const float4* np, float ox, float oy
     tg = make_uint2(__float_as_uint(n1.y), hitmask & 0x00FFFFFFu);
 }
 
+// Issue-bound like the flat kernel (306 warp instructions per primary ray at
+// 81 % of the issue slots before, 18 of 32 lanes at work).  What it measured on
+// the city of 625 instances, 4.2M primary rays closest-hit / one AO ray each
+// any-hit, us: 1,394 / 836 as it was; 1,362 / 806 with the world ray kept in
+// shared memory instead of read and inverted again on leaving an instance;
+// 1,294 / 798 with pairs of triangle tests as in the flat kernel and 72
+// registers, seven blocks per SM (64 and eight: 1,303 / 814; 80 and six: 1,353
+// / 841; 56 and nine spill: 1,411 / 845); 1,131 / 786 with refills at Nd 6 / Nw
+// 32 instead of 2 / 8 (4 / 16: 1,183 / 792), which keep a warp's camera rays
+// together.  Entering instances only when 4 or 8 lanes would: 3-6 % slower.
 template <bool ANY, int SMEM>
-__global__ void __launch_bounds__(128, 8) cwbvh_inst_kernel(const InstParams p) {
+__global__ void __launch_bounds__(128, 7) cwbvh_inst_kernel(const InstParams p) {
     extern __shared__ uint2 sstack[];
     constexpr int LOCAL = kInstStack - SMEM;
     uint2 lstack[LOCAL];
@@ -109,19 +119,30 @@ __global__ void __launch_bounds__(128, 8) cwbvh_inst_kernel(const InstParams p) 
         --sp;
         return sp < SMEM ? sstack[(unsigned)sp * B + tid] : lstack[sp - SMEM];
     };
+    auto set_octant = [&]() {
+        octinv = 7u - (((dx < 0.f) ? 4u : 0u) | ((dy < 0.f) ? 2u : 0u) | ((dz < 0.f) ? 1u : 0u));
+        octinv4 = octinv * 0x01010101u;
+    };
     auto set_ray = [&](float4 o, float4 d) {
         ox = o.x; oy = o.y; oz = o.z;
         dx = d.x; dy = d.y; dz = d.z;
         idx_ = guarded_rcp(dx);
         idy = guarded_rcp(dy);
         idz = guarded_rcp(dz);
-        octinv = 7u - (((dx < 0.f) ? 4u : 0u) | ((dy < 0.f) ? 2u : 0u) | ((dz < 0.f) ? 1u : 0u));
-        octinv4 = octinv * 0x01010101u;
+        set_octant();
     };
-    auto to_world = [&]() {
+    // The world ray, nine words per lane after the stacks.
+    float* const world = reinterpret_cast<float*>(sstack + SMEM * B) + tid;
+    auto top_level = [&]() {
         in_blas = false;
         nodes = p.tlas_nodes; woop = p.tlas_rows; node_f4 = p.tlas_node_f4; woop_f4 = p.tlas_rows_f4;
-        set_ray(__ldg(&p.rays[ray].origin_tmin), __ldg(&p.rays[ray].dir_tmax));
+    };
+    auto to_world = [&]() {
+        top_level();
+        ox = world[0]; oy = world[B]; oz = world[2 * B];
+        dx = world[3 * B]; dy = world[4 * B]; dz = world[5 * B];
+        idx_ = world[6 * B]; idy = world[7 * B]; idz = world[8 * B];
+        set_octant();
     };
     auto finish = [&](unsigned err) {
         if (err) {
@@ -146,9 +167,14 @@ __global__ void __launch_bounds__(128, 8) cwbvh_inst_kernel(const InstParams p) 
                 const int64_t g = (int64_t)base + __popc(needm & lanemask_lt());
                 if (g < p.total_rays) {
                     ray = g;
-                    to_world();
-                    tmin = __ldg(&p.rays[g].origin_tmin).w;
-                    tmax = __ldg(&p.rays[g].dir_tmax).w;
+                    const float4 o = __ldg(&p.rays[g].origin_tmin), d = __ldg(&p.rays[g].dir_tmax);
+                    top_level();
+                    set_ray(o, d);
+                    world[0] = ox; world[B] = oy; world[2 * B] = oz;
+                    world[3 * B] = dx; world[4 * B] = dy; world[5 * B] = dz;
+                    world[6 * B] = idx_; world[7 * B] = idy; world[8 * B] = idz;
+                    tmin = o.w;
+                    tmax = d.w;
                     ng = make_uint2(0u, 0x80000000u);
                     tg = make_uint2(0u, 0u);
                     sp = 0; inst_sp = 0; cur_inst = -1;
@@ -208,14 +234,24 @@ __global__ void __launch_bounds__(128, 8) cwbvh_inst_kernel(const InstParams p) 
                     }
                     const float4 r0 = ld_nc(woop + tri), r1 = ld_nc(woop + tri + 1), r2 = ld_nc(woop + tri + 2);
                     if (in_blas) {
-                        float t, u, v;
-                        if (woop_test(r0, r1, r2, ox, oy, oz, dx, dy, dz, tmin, tmax, t, u, v)) {
-                            tmax = t;
-                            hit_addr = (int)tri;
-                            hit_inst = cur_inst;
-                            hu = u;
-                            hv = v;
-                            if (ANY) finish(0u);
+                        auto test = [&](const float4& a, const float4& b, const float4& c, unsigned addr) {
+                            float t, u, v;
+                            if (woop_test(a, b, c, ox, oy, oz, dx, dy, dz, tmin, tmax, t, u, v)) {
+                                tmax = t;
+                                hit_addr = (int)addr;
+                                hit_inst = cur_inst;
+                                hu = u;
+                                hv = v;
+                                if (ANY) finish(0u);
+                            }
+                        };
+                        test(r0, r1, r2, tri);
+                        if (active && tg.y != 0u) {  // the lane's next triangle in the same round
+                            const unsigned ti2 = highest_bit(tg.y);
+                            const unsigned tri2 = tg.x * 3u + ti2 * 3u;
+                            tg.y &= ~(1u << ti2);
+                            if ((uint64_t)tri2 + 3u > (uint64_t)woop_f4) finish(kErrBadScene);
+                            else test(ld_nc(woop + tri2), ld_nc(woop + tri2 + 1), ld_nc(woop + tri2 + 2), tri2);
                         }
                         continue;
                     }
@@ -370,12 +406,12 @@ rq_status rq_trace_instanced(rq_ctx_t ctx, rq_tlas_t tlas, const rq_ray* rays, r
     // Postponing is off unless asked for: on the instanced city it measured
     // 2 % slower than the oracle's order (instance entries are postponed too).
     p.postpone_ratio = launch && launch->postpone_ratio > 0.f ? l.postpone_ratio : 0.f;
-    p.fetch_nd = l.fetch_nd;
-    p.fetch_nw = l.fetch_nw;
+    p.fetch_nd = launch && launch->fetch_nd != 0 ? l.fetch_nd : 6;   // measured at the kernel
+    p.fetch_nw = launch && launch->fetch_nw > 0 ? l.fetch_nw : 32;
     p.step_limit = l.step_limit;
     constexpr int kSmem = 8, kBlock = 128;
     void (*fn)(InstParams) = query == RQ_ANY ? cwbvh_inst_kernel<true, kSmem> : cwbvh_inst_kernel<false, kSmem>;
-    const size_t smem = (size_t)kSmem * kBlock * sizeof(uint2);
+    const size_t smem = (kSmem * sizeof(uint2) + 9 * sizeof(float)) * (size_t)kBlock;  // stacks, world rays
     int per_sm = 0;
     RQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kBlock, smem));
     const int64_t blocks_needed = (count + kBlock - 1) / kBlock;
