@@ -58,21 +58,6 @@ __device__ __forceinline__ void store_ray(Ray* r, float4 o, float4 d, bool wide)
 }
 static bool aligned32(const void* p) { return ((uintptr_t)p & 31u) == 0; }
 
-// Division of 31-bit numbers by one divisor: floor(i / d) = i * mul >> shift
-// with mul = ceil(2^shift / d) and shift = 31 + ceil(log2 d) is exact for every
-// i < 2^31 (Granlund and Montgomery, "Division by Invariant Integers using
-// Multiplication", PLDI 1994), mul < 2^32.
-struct FastDiv {
-    uint32_t mul, shift, d;
-    explicit FastDiv(uint32_t divisor) : d(divisor) {
-        uint32_t l = 0;
-        while (l < 31 && (1ull << l) < divisor) ++l;
-        shift = 31 + l;
-        mul = (uint32_t)(((1ull << shift) + divisor - 1) / divisor);
-    }
-    __device__ uint32_t div(uint32_t i) const { return (uint32_t)((uint64_t)i * mul >> shift); }
-};
-
 // Surfel frame in shared memory: normal, tangents, ray origin.
 struct SurfelFrame {
     float3 n, t1, t2, o;
@@ -93,12 +78,11 @@ constexpr int kAoBlock = 256;
 // block's rays start `skip` samples into its first surfel.  16M rays at 4 per
 // surfel 199 -> 159 us, 1M at 32 per surfel 16.6 -> 12.7 us, the same bits.
 template <bool SMALL>
-__global__ void __launch_bounds__(kAoBlock) aorays_kernel(
-        const float4* __restrict__ pos, const float4* __restrict__ nrm, const float* __restrict__ radius,
-        int64_t n_rays, FastDiv spp, int64_t first_ray, uint32_t k0, uint32_t k1, float tmin, float tmax,
-        float offset_scale, Ray* __restrict__ out, bool wide) {
-    __shared__ SurfelFrame frames[kAoBlock];
-    const int64_t block0 = (int64_t)blockIdx.x * kAoBlock;
+__device__ __forceinline__ void aorays_block(
+        SurfelFrame* frames, int64_t block, const float4* __restrict__ pos, const float4* __restrict__ nrm,
+        const float* __restrict__ radius, int64_t n_rays, FastDiv spp, int64_t first_ray, uint32_t k0, uint32_t k1,
+        float tmin, float tmax, float offset_scale, Ray* __restrict__ out, bool wide, uint32_t* __restrict__ counts) {
+    const int64_t block0 = block * kAoBlock;
     const int64_t surfel0 = SMALL ? (int64_t)spp.div((uint32_t)block0) : block0 / spp.d;  // SMALL: n_rays < 2^31
     const uint32_t skip = (uint32_t)(block0 - surfel0 * spp.d);
     const uint32_t here = (uint32_t)(n_rays - block0 < kAoBlock ? n_rays - block0 : kAoBlock);  // rays of the block
@@ -106,6 +90,7 @@ __global__ void __launch_bounds__(kAoBlock) aorays_kernel(
     const uint32_t n_surfels = spp.div(skip + here - 1u) + 1u;
     if (threadIdx.x < n_surfels) {
         const int64_t s = surfel0 + threadIdx.x;
+        if (counts && (threadIdx.x > 0 || skip == 0)) counts[s] = 0u;  // the block of a surfel's first ray
         const float3 p = f3(pos[s]);
         const float3 n = f3(nrm[s]);
         const float r = radius ? radius[s] : 0.0f;
@@ -147,6 +132,42 @@ __global__ void __launch_bounds__(kAoBlock) aorays_kernel(
     const float dzl = sqrtf(fmaxf(0.0f, 1.0f - dxl * dxl - dyl * dyl));
     const float3 d = norm3(add3(add3(mul3(f.t1, dxl), mul3(f.t2, dyl)), mul3(n, dzl)));
     store_ray(out + i, make_float4(o.x, o.y, o.z, tmin), make_float4(d.x, d.y, d.z, tmax), wide);
+}
+
+template <bool SMALL>
+__global__ void __launch_bounds__(kAoBlock) aorays_kernel(
+        const float4* __restrict__ pos, const float4* __restrict__ nrm, const float* __restrict__ radius,
+        int64_t n_rays, FastDiv spp, int64_t first_ray, uint32_t k0, uint32_t k1, float tmin, float tmax,
+        float offset_scale, Ray* __restrict__ out, bool wide) {
+    __shared__ SurfelFrame frames[kAoBlock];
+    aorays_block<SMALL>(frames, blockIdx.x, pos, nrm, radius, n_rays, spp, first_ray, k0, k1, tmin, tmax, offset_scale,
+                        out, wide, nullptr);
+}
+
+// The pieces of a bake launch together: a block finds its piece by its number.
+template <class Begin>
+__device__ __forceinline__ int item_of_block(const AoItem* items, int n_items, Begin begin) {
+    int lo = 0, hi = n_items - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (begin(items[mid]) <= blockIdx.x) lo = mid; else hi = mid - 1;
+    }
+    return lo;
+}
+
+__global__ void __launch_bounds__(kAoBlock) aorays_items_kernel(const AoItem* __restrict__ items, int n_items) {
+    __shared__ SurfelFrame frames[kAoBlock];
+    const AoItem& it = items[item_of_block(items, n_items, [](const AoItem& i) { return i.block_begin; })];
+    aorays_block<true>(frames, blockIdx.x - it.block_begin, it.pos, it.nrm, it.radius, it.n_rays, it.spp, it.first_ray,
+                       it.k0, it.k1, it.tmin, it.tmax, it.offset_scale, it.rays, it.wide != 0u, it.counts);
+}
+
+// Occluded-ray counts turned into AO fractions (at the counters themselves or
+// in mapped host memory).
+__global__ void __launch_bounds__(kAoBlock) ao_finish_items_kernel(const AoItem* __restrict__ items, int n_items) {
+    const AoItem& it = items[item_of_block(items, n_items, [](const AoItem& i) { return i.surfel_block_begin; })];
+    const int64_t i = (int64_t)(blockIdx.x - it.surfel_block_begin) * kAoBlock + threadIdx.x;
+    if (i < it.n_surfels) it.ao[i] = (float)it.counts[i] / (float)(int)it.spp.d;
 }
 
 // Surfel i on triangle floor(u * nt) at barycentrics (1 - sqrt(a), b sqrt(a)).
@@ -367,6 +388,23 @@ rq_status aorays_launch(const float* pos, const float* nrm, const float* radius,
     kernel<<<blocks_for(n, kAoBlock), kAoBlock, 0, (cudaStream_t)stream>>>(
         (const float4*)pos, (const float4*)nrm, radius, n, FastDiv((uint32_t)spp), first_ray, (uint32_t)seed, (uint32_t)(seed >> 32),
         tmin, tmax, offset_scale, (Ray*)out_rays, aligned32(out_rays));
+    RQ_CUDA(cudaGetLastError());
+    return RQ_OK;
+}
+
+uint32_t ao_ray_blocks(int64_t n_rays) { return blocks_for(n_rays, kAoBlock); }
+uint32_t ao_surfel_blocks(int64_t n_surfels) { return blocks_for(n_surfels, kAoBlock); }
+
+rq_status aorays_items_launch(const AoItem* items, int n_items, uint32_t blocks, cudaStream_t s) {
+    if (blocks == 0) return RQ_OK;
+    aorays_items_kernel<<<blocks, kAoBlock, 0, s>>>(items, n_items);
+    RQ_CUDA(cudaGetLastError());
+    return RQ_OK;
+}
+
+rq_status ao_finish_items_launch(const AoItem* items, int n_items, uint32_t blocks, cudaStream_t s) {
+    if (blocks == 0) return RQ_OK;
+    ao_finish_items_kernel<<<blocks, kAoBlock, 0, s>>>(items, n_items);
     RQ_CUDA(cudaGetLastError());
     return RQ_OK;
 }

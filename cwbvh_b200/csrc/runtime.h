@@ -76,6 +76,47 @@ rq_status aorays_launch(const float* pos, const float* nrm, const float* radius,
                         int64_t first_ray, uint64_t seed, float tmin, float tmax, float offset_scale, rq_ray* out_rays,
                         void* stream);
 
+// Division of 31-bit numbers by one divisor: floor(i / d) = i * mul >> shift
+// with mul = ceil(2^shift / d) and shift = 31 + ceil(log2 d) is exact for every
+// i < 2^31 (Granlund and Montgomery, "Division by Invariant Integers using
+// Multiplication", PLDI 1994), mul < 2^32.
+struct FastDiv {
+    uint32_t mul, shift, d;
+    explicit FastDiv(uint32_t divisor) : d(divisor) {
+        uint32_t l = 0;
+        while (l < 31 && (1ull << l) < divisor) ++l;
+        shift = 31 + l;
+        mul = (uint32_t)(((1ull << shift) + divisor - 1) / divisor);
+    }
+    __device__ uint32_t div(uint32_t i) const { return (uint32_t)((uint64_t)i * mul >> shift); }
+};
+
+// AO bake work of one launch over several pieces (rays.cu): piece k's rays are
+// made by blocks [block_begin, next piece's), which also zero its counters;
+// the counters then become AO fractions at `ao`.  Inputs and `ao` are device
+// addresses, of device memory or of mapped host memory.
+struct AoItem {
+    const float4* pos;
+    const float4* nrm;
+    const float* radius;
+    Ray* rays;
+    uint32_t* counts;
+    float* ao;
+    int64_t first_ray;
+    int64_t n_surfels;
+    FastDiv spp;
+    uint32_t n_rays;  // below 2^31
+    uint32_t k0, k1;
+    float tmin, tmax, offset_scale;
+    uint32_t block_begin;         // of the ray launch
+    uint32_t surfel_block_begin;  // of the AO launch
+    uint32_t wide;                // rays 32-byte aligned
+};
+uint32_t ao_ray_blocks(int64_t n_rays);      // blocks of a piece in the ray launch
+uint32_t ao_surfel_blocks(int64_t n_surfels);  // and in the AO launch
+rq_status aorays_items_launch(const AoItem* items, int n_items, uint32_t blocks, cudaStream_t s);
+rq_status ao_finish_items_launch(const AoItem* items, int n_items, uint32_t blocks, cudaStream_t s);
+
 // Morton keys + radix sort of the rays of several items (rays.cu).
 struct SortPlan {
     int n_items = 0;
