@@ -46,12 +46,19 @@ struct TraceItem {
     const int32_t* perm;
     int64_t ray_begin;
     int64_t count;
-    uint32_t node_f4;  // node buffer length in float4 (bounds checks)
-    uint32_t woop_f4;  // Woop buffer length in float4
+    // Bounds checks: addresses from these on leave the buffers (trace.cu).
+    uint32_t node_limit;  // CWBVH: nodes; BVH2: float4 addresses with a whole node behind them
+    uint32_t woop_limit;  // CWBVH: addresses with three rows behind them; BVH2: float4 of the buffer
     uint32_t* ao_counts;  // non-null: occluded rays are counted per surfel here instead of writing hits
     int32_t ao_spp;       // rays per surfel (consecutive) when ao_counts is set
     int32_t pad;
 };
+
+// Limits of a buffer of f4 float4 (at most UINT32_MAX): whole records in it,
+// and addresses with `rows` float4 behind them.  A kernel then checks an
+// address with one 32-bit compare instead of a 64-bit sum and compare.
+inline uint32_t record_limit(int64_t f4, int64_t record) { return (uint32_t)(f4 / record); }
+inline uint32_t address_limit(int64_t f4, int64_t rows) { return f4 >= rows ? (uint32_t)(f4 - rows + 1) : 0u; }
 
 struct TraceParams {
     TraceItem single;         // the scene when the kernel is not a batch kernel

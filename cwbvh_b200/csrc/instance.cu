@@ -28,15 +28,15 @@ namespace rq {
 struct BlasDesc {
     const float4* nodes;
     const float4* woop;
-    uint32_t node_f4;
-    uint32_t woop_f4;
+    uint32_t node_limit;  // nodes
+    uint32_t woop_limit;  // addresses whose three rows are inside the buffer
 };
 
 struct InstParams {
     const float4* tlas_nodes;
     const float4* tlas_rows;    // 3 float4 per instance slot: world-to-object rows
     const int32_t* tlas_map;    // (instance, blas, -1) per row
-    uint32_t tlas_node_f4, tlas_rows_f4;
+    uint32_t tlas_node_limit, tlas_rows_limit;
     const BlasDesc* blas;
     int n_blas;
     const Ray* rays;
@@ -67,7 +67,7 @@ __device__ __forceinline__ void cwbvh_visit(const float4* np, float ox, float oy
     const float orx = __fmul_rn(-__fsub_rn(ox, n0.x), idx_);
     const float ory = __fmul_rn(-__fsub_rn(oy, n0.y), idy);
     const float orz = __fmul_rn(-__fsub_rn(oz, n0.z), idz);
-    const unsigned hitmask = cwbvh_hitmask(n1, n2, n3, n4, adjx, adjy, adjz, orx, ory, orz, idx_ < 0.f, idy < 0.f,
+    const unsigned hitmask = cwbvh_hitmask<false>(n1, n2, n3, n4, adjx, adjy, adjz, orx, ory, orz, idx_ < 0.f, idy < 0.f,
                                            idz < 0.f, octinv4, tmin, tmax);
     ng = make_uint2(__float_as_uint(n1.x), (hitmask & 0xFF000000u) | (ew >> 24));
     tg = make_uint2(__float_as_uint(n1.y), hitmask & 0x00FFFFFFu);
@@ -82,7 +82,8 @@ __device__ __forceinline__ void cwbvh_visit(const float4* np, float ox, float oy
 // registers, seven blocks per SM (64 and eight: 1,303 / 814; 80 and six: 1,353
 // / 841; 56 and nine spill: 1,411 / 845); 1,131 / 786 with refills at Nd 6 / Nw
 // 32 instead of 2 / 8 (4 / 16: 1,183 / 792), which keep a warp's camera rays
-// together.  Entering instances only when 4 or 8 lanes would: 3-6 % slower.
+// together; 1,115 / 777 with 32-bit limits and branch-free triangle
+// acceptance.  Entering instances only when 4 or 8 lanes would: 3-6 % slower.
 template <bool ANY, int SMEM>
 __global__ void __launch_bounds__(128, 7) cwbvh_inst_kernel(const InstParams p) {
     extern __shared__ uint2 sstack[];
@@ -95,7 +96,7 @@ __global__ void __launch_bounds__(128, 7) cwbvh_inst_kernel(const InstParams p) 
     // current level: the top-level tree, or the BLAS of instance `cur_inst`
     const float4* nodes = p.tlas_nodes;
     const float4* woop = p.tlas_rows;
-    uint32_t node_f4 = p.tlas_node_f4, woop_f4 = p.tlas_rows_f4;
+    uint32_t node_limit = p.tlas_node_limit, woop_limit = p.tlas_rows_limit;
     bool in_blas = false;
     int inst_sp = 0, cur_inst = -1;
 
@@ -135,7 +136,7 @@ __global__ void __launch_bounds__(128, 7) cwbvh_inst_kernel(const InstParams p) 
     float* const world = reinterpret_cast<float*>(sstack + SMEM * B) + tid;
     auto top_level = [&]() {
         in_blas = false;
-        nodes = p.tlas_nodes; woop = p.tlas_rows; node_f4 = p.tlas_node_f4; woop_f4 = p.tlas_rows_f4;
+        nodes = p.tlas_nodes; woop = p.tlas_rows; node_limit = p.tlas_node_limit; woop_limit = p.tlas_rows_limit;
     };
     auto to_world = [&]() {
         top_level();
@@ -201,7 +202,7 @@ __global__ void __launch_bounds__(128, 7) cwbvh_inst_kernel(const InstParams p) 
                     const unsigned slot = (bit - 24u) ^ octinv;
                     const unsigned ci = base + (unsigned)__popc(hitsm & ~(0xFFFFFFFFu << slot));
                     if (++steps > p.step_limit) fault |= kErrTimeout;
-                    if ((uint64_t)ci * 5u + 5u > (uint64_t)node_f4) fault |= kErrBadScene;
+                    if (ci >= node_limit) fault |= kErrBadScene;
                     if (!fault) cwbvh_visit(nodes + (size_t)ci * 5u, ox, oy, oz, idx_, idy, idz, octinv4, tmin, tmax,
                                             ng, tg);
                 } else {
@@ -228,7 +229,7 @@ __global__ void __launch_bounds__(128, 7) cwbvh_inst_kernel(const InstParams p) 
                     const unsigned ti = highest_bit(tg.y);
                     const unsigned tri = tg.x * 3u + ti * 3u;
                     tg.y &= ~(1u << ti);
-                    if ((uint64_t)tri + 3u > (uint64_t)woop_f4) {
+                    if (tri >= woop_limit) {
                         finish(kErrBadScene);
                         continue;
                     }
@@ -250,7 +251,7 @@ __global__ void __launch_bounds__(128, 7) cwbvh_inst_kernel(const InstParams p) 
                             const unsigned ti2 = highest_bit(tg.y);
                             const unsigned tri2 = tg.x * 3u + ti2 * 3u;
                             tg.y &= ~(1u << ti2);
-                            if ((uint64_t)tri2 + 3u > (uint64_t)woop_f4) finish(kErrBadScene);
+                            if (tri2 >= woop_limit) finish(kErrBadScene);
                             else test(ld_nc(woop + tri2), ld_nc(woop + tri2 + 1), ld_nc(woop + tri2 + 2), tri2);
                         }
                         continue;
@@ -279,7 +280,7 @@ __global__ void __launch_bounds__(128, 7) cwbvh_inst_kernel(const InstParams p) 
                         __fmaf_rn(r2.z, dz, __fmaf_rn(r2.y, dy, __fmul_rn(r2.x, dx))), 0.f);
                     set_ray(o, d);
                     const BlasDesc bd = p.blas[b];
-                    nodes = bd.nodes; woop = bd.woop; node_f4 = bd.node_f4; woop_f4 = bd.woop_f4;
+                    nodes = bd.nodes; woop = bd.woop; node_limit = bd.node_limit; woop_limit = bd.woop_limit;
                     ng = make_uint2(0u, 0x80000000u);
                     tg = make_uint2(0u, 0u);
                 }
@@ -342,8 +343,8 @@ rq_status rq_tlas_create(const rq_scene_t* blas, int n_blas, const float* object
         if (st != RQ_OK) return st;
         std::vector<BlasDesc> desc((size_t)n_blas);
         for (int b = 0; b < n_blas; ++b)
-            desc[(size_t)b] = BlasDesc{blas[b]->nodes, blas[b]->woop, (uint32_t)blas[b]->node_f4,
-                                       (uint32_t)blas[b]->woop_f4};
+            desc[(size_t)b] = BlasDesc{blas[b]->nodes, blas[b]->woop, record_limit(blas[b]->node_f4, 5),
+                                       address_limit(blas[b]->woop_f4, 3)};
         cudaError_t e = cudaMalloc(&t->d_blas, sizeof(BlasDesc) * (size_t)n_blas);
         if (e == cudaSuccess)
             e = cudaMemcpy(t->d_blas, desc.data(), sizeof(BlasDesc) * (size_t)n_blas, cudaMemcpyHostToDevice);
@@ -393,8 +394,8 @@ rq_status rq_trace_instanced(rq_ctx_t ctx, rq_tlas_t tlas, const rq_ray* rays, r
     p.tlas_nodes = top->nodes;
     p.tlas_rows = top->woop;
     p.tlas_map = top->prim_index;
-    p.tlas_node_f4 = (uint32_t)top->node_f4;
-    p.tlas_rows_f4 = (uint32_t)top->woop_f4;
+    p.tlas_node_limit = record_limit(top->node_f4, 5);
+    p.tlas_rows_limit = address_limit(top->woop_f4, 3);
     p.blas = tlas->d_blas;
     p.n_blas = tlas->n_blas;
     p.rays = (const Ray*)rays;

@@ -164,8 +164,11 @@ TraceItem scene_item(const rq_scene* sc, const rq_ray* rays, rq_hit* hits, int64
     it.perm = nullptr;
     it.ray_begin = 0;
     it.count = count;
-    it.node_f4 = (uint32_t)std::min<int64_t>(sc->node_f4, UINT32_MAX);
-    it.woop_f4 = (uint32_t)std::min<int64_t>(sc->woop_f4, UINT32_MAX);
+    const int64_t node_f4 = std::min<int64_t>(sc->node_f4, UINT32_MAX);
+    const int64_t woop_f4 = std::min<int64_t>(sc->woop_f4, UINT32_MAX);
+    const bool cw = sc->kind == RQ_BVH_CWBVH;
+    it.node_limit = cw ? record_limit(node_f4, 5) : address_limit(node_f4, 4);
+    it.woop_limit = cw ? address_limit(woop_f4, 3) : (uint32_t)woop_f4;
     return it;
 }
 

@@ -96,7 +96,7 @@ struct Lane {
     int64_t out_idx;
     int64_t gidx;
     int item;  // batch item of the ray (its hit buffer or AO counters are read at the end)
-    uint32_t node_f4, woop_f4;
+    uint32_t node_limit, woop_limit;
 };
 
 // Points a lane at global ray g of batch item `item` (0 for a single scene)
@@ -108,8 +108,8 @@ __device__ __forceinline__ const TraceItem* set_lane(const TraceParams& p, int64
     L.item = item;
     L.nodes = it->nodes;
     L.woop = it->woop;
-    L.node_f4 = it->node_f4;
-    L.woop_f4 = it->woop_f4;
+    L.node_limit = it->node_limit;
+    L.woop_limit = it->woop_limit;
     L.out_idx = it->perm ? (int64_t)__ldg(it->perm + local) : local;
     L.gidx = g;
     return it;
@@ -297,7 +297,7 @@ __global__ void RQ_KERNEL_BOUNDS cwbvh_kernel(const TraceParams p) {
                 const unsigned slot = (bit - 24u) ^ octinv;
                 const unsigned ci = base + (unsigned)__popc(hitsm & ~(0xFFFFFFFFu << slot));
                 if (++steps > p.step_limit) fault |= kErrTimeout;
-                if ((uint64_t)ci * 5u + 5u > (uint64_t)L.node_f4) fault |= kErrBadScene;
+                if (ci >= L.node_limit) fault |= kErrBadScene;
                 if (!fault) {
                     const float4* np = L.nodes + (size_t)ci * 5u;
                     const float4 n0 = ld_nc(np + 0), n1 = ld_nc(np + 1), n2 = ld_nc(np + 2);
@@ -311,7 +311,7 @@ __global__ void RQ_KERNEL_BOUNDS cwbvh_kernel(const TraceParams p) {
                     const float ory = __fmul_rn(-__fsub_rn(oy, n0.y), idy);
                     const float orz = __fmul_rn(-__fsub_rn(oz, n0.z), idz);
                     const bool negx = idx_ < 0.f, negy = idy < 0.f, negz = idz < 0.f;
-                    const unsigned hitmask = cwbvh_hitmask(n1, n2, n3, n4, adjx, adjy, adjz, orx, ory, orz, negx,
+                    const unsigned hitmask = cwbvh_hitmask<ANY>(n1, n2, n3, n4, adjx, adjy, adjz, orx, ory, orz, negx,
                                                            negy, negz, octinv4, tmin, tmax);
                     ng = make_uint2(__float_as_uint(n1.x), (hitmask & 0xFF000000u) | (ew >> 24));
                     tg = make_uint2(__float_as_uint(n1.y), hitmask & 0x00FFFFFFu);
@@ -379,7 +379,7 @@ __global__ void RQ_KERNEL_BOUNDS cwbvh_kernel(const TraceParams p) {
                             tri2 = tg.x * 3u + ti2 * 3u;
                             tg.y &= ~(1u << ti2);
                         }
-                        if ((uint64_t)tri + 3u > (uint64_t)L.woop_f4) {
+                        if (tri >= L.woop_limit) {
                             finish(kErrBadScene);
                         } else {
                             const float4* tp = L.woop + tri;
@@ -394,7 +394,7 @@ __global__ void RQ_KERNEL_BOUNDS cwbvh_kernel(const TraceParams p) {
                                 if (ANY) finish(0u);
                             }
                             if (two && active) {
-                                if ((uint64_t)tri2 + 3u > (uint64_t)L.woop_f4) {
+                                if (tri2 >= L.woop_limit) {
                                     finish(kErrBadScene);
                                 } else {
                                     const float4* tp2 = L.woop + tri2;
@@ -505,7 +505,7 @@ __global__ void __launch_bounds__(kLanesBlock) cwbvh_lanes_kernel(const TracePar
             const unsigned slot = (bit - 24u) ^ octinv;
             const unsigned ci = base + (unsigned)__popc(hitsm & ~(0xFFFFFFFFu << slot));
             if (++steps > p.step_limit) fault |= kErrTimeout;
-            if ((uint64_t)ci * 5u + 5u > (uint64_t)L.node_f4) fault |= kErrBadScene;
+            if (ci >= L.node_limit) fault |= kErrBadScene;
             if (!fault) {
                 const float4* np = L.nodes + (size_t)ci * 5u;
                 const float4 n0 = ld_nc(np + 0), n1 = ld_nc(np + 1), n2 = ld_nc(np + 2);
@@ -573,7 +573,7 @@ __global__ void __launch_bounds__(kLanesBlock) cwbvh_lanes_kernel(const TracePar
                 const unsigned ti = highest_bit(leaf_bits);
                 leaf_bits &= ~(1u << ti);
                 const unsigned tri = tri_base * 3u + ti * 3u;
-                if ((uint64_t)tri + 3u > (uint64_t)L.woop_f4) {
+                if (tri >= L.woop_limit) {
                     bad = true;
                     if (order < 0 || !ANY) order = (int)ti;
                     break;
@@ -735,7 +735,7 @@ __global__ void RQ_BVH2_BOUNDS bvh2_kernel(const TraceParams p) {
                 if (in) {
                     unsigned fault = 0u;
                     if (++steps > p.step_limit) fault |= kErrTimeout;
-                    if ((uint64_t)(unsigned)node + 4u > (uint64_t)L.node_f4) fault |= kErrBadScene;
+                    if ((unsigned)node >= L.node_limit) fault |= kErrBadScene;
                     if (!fault) {
                         const float4* np = L.nodes + node;
                         const float4 n0 = ld_nc(np), n1 = ld_nc(np + 1), n2 = ld_nc(np + 2), n3 = ld_nc(np + 3);
@@ -778,7 +778,7 @@ __global__ void RQ_BVH2_BOUNDS bvh2_kernel(const TraceParams p) {
                 const bool want = active && leaf < 0;
                 if (__ballot_sync(kFullMask, want) == 0u) break;
                 if (want) {
-                    if ((uint64_t)(unsigned)tcur + 1u > (uint64_t)L.woop_f4) {
+                    if ((unsigned)tcur >= L.woop_limit) {
                         finish(kErrBadScene);
                     } else {
                         const float4 v0 = ld_nc(L.woop + tcur);
@@ -789,7 +789,7 @@ __global__ void RQ_BVH2_BOUNDS bvh2_kernel(const TraceParams p) {
                                 node = pop();
                                 tcur = ~leaf;
                             }
-                        } else if ((uint64_t)(unsigned)tcur + 3u > (uint64_t)L.woop_f4) {
+                        } else if (L.woop_limit - (unsigned)tcur < 3u) {
                             finish(kErrBadScene);
                         } else {
                             const float4 v1 = ld_nc(L.woop + tcur + 1), v2 = ld_nc(L.woop + tcur + 2);
