@@ -119,7 +119,7 @@ rq_status rq_batch_run(rq_batch_t b, void* stream) {
     cudaStream_t s = (cudaStream_t)stream;
     if (!b->params.use_graph || s == nullptr) return batch_enqueue(b, s);
     if (!b->exec) {
-        warm_launch_cache(b->kind, b->query, b->launch, true, false);
+        warm_launch_cache(b->kind, b->query, b->launch, true, false, b->free_shape);
         RQ_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeRelaxed));
         rq_status st = batch_enqueue(b, s);
         cudaGraph_t g = nullptr;

@@ -89,6 +89,6 @@ TraceKernelFn trace_kernel(rq_bvh_kind kind, bool any, int smem, bool multi, boo
 TraceKernelFn lanes_kernel(bool any, bool multi, int g);
 int lanes_block();
 int smem_entries_of(int requested);
-size_t trace_smem_bytes(rq_bvh_kind kind, int smem_entries, int block, bool ring);
+size_t trace_smem_bytes(rq_bvh_kind kind, int smem_entries, int block, bool multi, bool ring);
 
 }  // namespace rq

@@ -101,16 +101,24 @@ static int lanes_per_ray(rq_query q, int64_t rays, int sms) {
     return rays <= (q == RQ_ANY ? 448 : 320) * (int64_t)sms ? 4 : 0;
 }
 
+// Stack entries per lane in shared memory of the ring kernels where the caller
+// leaves the shape open: nine blocks with rings and eight entries leave L1 28 KB
+// (18M AO rays of 12 scenes 3,370 us), with four 60 KB (3,205 us).  The kernels
+// without rings are the same within 1 % from 4 to 16.  A refill from the ring
+// is cheap, so they also refill sooner, at Nw 4 instead of 8 (3,178 us; the
+// others lose 1 % by it).
+constexpr int kRingStack = 4, kRingFetchNw = 4;
+
 rq_status launch_trace(rq_bvh_kind kind, rq_query q, const rq_launch& l, bool multi, bool count, bool free_shape,
                        const TraceParams& p, cudaStream_t s) {
     if (p.total_rays <= 0) return RQ_OK;
-    void* args[] = {(void*)&p};
     int dev = 0;
     RQ_CUDA(cudaGetDevice(&dev));
     if (free_shape && kind == RQ_BVH_CWBVH && !count) {
         if (const int g = lanes_per_ray(q, p.total_rays, device_sms(dev))) {
             const int64_t rays_per_block = lanes_block() / g;
             const unsigned blocks = (unsigned)((p.total_rays + rays_per_block - 1) / rays_per_block);
+            void* args[] = {(void*)&p};
             RQ_CUDA(cudaLaunchKernel((const void*)lanes_kernel(q == RQ_ANY, multi, g), dim3(blocks),
                                      dim3((unsigned)lanes_block()), args, 0, s));
             return RQ_OK;
@@ -118,14 +126,17 @@ rq_status launch_trace(rq_bvh_kind kind, rq_query q, const rq_launch& l, bool mu
     }
     RQ_CUDA(cudaMemsetAsync(&p.scratch->ray_counter, 0, sizeof(unsigned long long), s));
     // Any-hit launches with many rays per thread take the ring-prefetching kernel.
+    TraceParams tp = p;
     TraceKernelFn fn = nullptr;
     size_t smem = 0;
     int nb = 1;
     auto pick = [&](bool ring) {
-        fn = trace_kernel(kind, q == RQ_ANY, l.smem_stack, multi, count, ring);
-        smem = trace_smem_bytes(kind, smem_entries_of(l.smem_stack), l.block_size, ring);
+        const int stack = ring && free_shape ? kRingStack : l.smem_stack;
+        fn = trace_kernel(kind, q == RQ_ANY, stack, multi, count, ring);
+        smem = trace_smem_bytes(kind, smem_entries_of(stack), l.block_size, multi, ring);
         nb = blocks_per_sm(fn, l.block_size, smem);
         if (l.blocks_per_sm > 0) nb = std::min(nb, l.blocks_per_sm);
+        tp.fetch_nw = ring && free_shape ? kRingFetchNw : p.fetch_nw;
     };
     const bool ring = kind == RQ_BVH_CWBVH && !count && q == RQ_ANY;
     pick(ring);
@@ -137,14 +148,16 @@ rq_status launch_trace(rq_bvh_kind kind, rq_query q, const rq_launch& l, bool mu
     const int64_t warps_needed = (p.total_rays + 31) / 32;
     const int64_t blocks_needed = (warps_needed * 32 + l.block_size - 1) / l.block_size;
     grid = std::max<int64_t>(1, std::min(grid, blocks_needed));
+    void* args[] = {(void*)&tp};
     RQ_CUDA(cudaLaunchKernel((const void*)fn, dim3((unsigned)grid), dim3((unsigned)l.block_size), args, smem, s));
     return RQ_OK;
 }
 
-void warm_launch_cache(rq_bvh_kind kind, rq_query q, const rq_launch& l, bool multi, bool count) {
+void warm_launch_cache(rq_bvh_kind kind, rq_query q, const rq_launch& l, bool multi, bool count, bool free_shape) {
     for (int ring = 0; ring <= (kind == RQ_BVH_CWBVH && !count && q == RQ_ANY ? 1 : 0); ++ring) {
-        TraceKernelFn fn = trace_kernel(kind, q == RQ_ANY, l.smem_stack, multi, count, ring != 0);
-        blocks_per_sm(fn, l.block_size, trace_smem_bytes(kind, smem_entries_of(l.smem_stack), l.block_size, ring != 0));
+        const int stack = ring && free_shape ? kRingStack : l.smem_stack;
+        TraceKernelFn fn = trace_kernel(kind, q == RQ_ANY, stack, multi, count, ring != 0);
+        blocks_per_sm(fn, l.block_size, trace_smem_bytes(kind, smem_entries_of(stack), l.block_size, multi, ring != 0));
     }
     int dev = 0;
     if (cudaGetDevice(&dev) == cudaSuccess) device_sms(dev);

@@ -62,7 +62,7 @@ rq_status launch_trace(rq_bvh_kind kind, rq_query q, const rq_launch& l, bool mu
                        const TraceParams& p, cudaStream_t s);
 
 // Computes the occupancy of a kernel variant ahead of a stream capture.
-void warm_launch_cache(rq_bvh_kind kind, rq_query q, const rq_launch& l, bool multi, bool count);
+void warm_launch_cache(rq_bvh_kind kind, rq_query q, const rq_launch& l, bool multi, bool count, bool free_shape);
 
 // Zeroes the context's ray counter on the stream.
 rq_status reset_counter(rq_ctx* ctx, cudaStream_t s);

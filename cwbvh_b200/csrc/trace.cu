@@ -29,10 +29,10 @@ constexpr int kStackTotal = 64;  // entries per lane (shared + local)
 constexpr int kDeeperMinLanes = 16;  // any-hit: lanes that make a second node step worth its issue slots
 
 #ifdef RQ_MAXNREG
-#define RQ_KERNEL_BOUNDS __maxnreg__(RQ_MAXNREG)  // register cap (occupancy experiments)
+#define RQ_CW_BOUNDS __maxnreg__(RQ_MAXNREG)  // register cap (occupancy experiments)
 #define RQ_BVH2_BOUNDS __maxnreg__(RQ_MAXNREG)
 #else
-#define RQ_KERNEL_BOUNDS __launch_bounds__(512)
+#define RQ_CW_BOUNDS __maxnreg__(COUNT ? 64 : 56)  // see park_bytes_per_warp
 // The BVH2 kernel fits 56 registers without spilling (nine 128-thread blocks
 // per SM instead of eight): closest-hit +2.3 %, any-hit unchanged on the
 // small scene; 48 spills and loses 2 % any-hit.
@@ -63,6 +63,21 @@ constexpr unsigned kRingSlots = 2 * kRingHalf;
 // rays [64][2] float4, the two halves' first global ray index, items [64]
 constexpr size_t kRingBytesPerWarp = kRingSlots * sizeof(Ray) + 2 * sizeof(int64_t) + kRingSlots * sizeof(int);
 static_assert(kRingBytesPerWarp % 16 == 0, "ring keeps 16 B alignment");
+
+// A CWBVH ray's values that only its end or a rare branch reads wait in shared
+// memory, a word per lane each: hit address, u, v, result index (two words),
+// and for a batch its item, the prefetched item and the item's Woop limit.  With
+// them in registers the kernels took 64 and eight 128-thread blocks fit an SM;
+// without, 56 and nine, with no spills (10 B in the ring batch kernel with more
+// than four stack entries; 72 registers and seven blocks are 1-6 % slower than 64, 48 and ten spill and
+// are 2-10 % slower).  Single-scene kernels read the limits from the launch
+// parameters.  4.2M city primary rays 808 -> 795 us, 4M AO rays on 4M triangles
+// 1,240 -> 1,204 us, 1M closest hits 390 -> 389 us, 18M AO rays of 12 scenes
+// 3,332 -> 3,205 us (with four stack entries, see launch_trace).
+constexpr int kParkWordsSingle = 5, kParkWordsMulti = 8;
+__host__ __device__ constexpr size_t park_bytes_per_warp(bool multi) {
+    return (multi ? kParkWordsMulti : kParkWordsSingle) * 32 * sizeof(int);
+}
 
 __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc) {
     const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
@@ -135,20 +150,25 @@ __device__ __forceinline__ void store_hit(Hit* hits, int64_t i, float t, int add
 // A finished ray's result: its Hit, or -- for an item with AO counters -- one
 // count for its surfel when it is occluded.
 template <bool MULTI>
-__device__ __forceinline__ void finish_ray(const TraceParams& p, const Lane& L, float t, int addr, float u, float v) {
-    const TraceItem* it = MULTI ? p.items + L.item : &p.single;
+__device__ __forceinline__ void finish_ray(const TraceParams& p, int item, int64_t out_idx, float t, int addr, float u,
+                                           float v) {
+    const TraceItem* it = MULTI ? p.items + item : &p.single;
     uint32_t* counts = it->ao_counts;
     if (counts) {
-        if (addr >= 0) atomicAdd(counts + L.out_idx / it->ao_spp, 1u);
+        if (addr >= 0) atomicAdd(counts + out_idx / it->ao_spp, 1u);
     } else {
-        store_hit(it->hits, L.out_idx, t, addr, u, v);
+        store_hit(it->hits, out_idx, t, addr, u, v);
     }
+}
+template <bool MULTI>
+__device__ __forceinline__ void finish_ray(const TraceParams& p, const Lane& L, float t, int addr, float u, float v) {
+    finish_ray<MULTI>(p, L.item, L.out_idx, t, addr, u, v);
 }
 
 // ------------------------------------------------------------------ CWBVH --
 
 template <bool ANY, int SMEM, bool MULTI, bool COUNT, bool RING>
-__global__ void RQ_KERNEL_BOUNDS cwbvh_kernel(const TraceParams p) {
+__global__ void RQ_CW_BOUNDS cwbvh_kernel(const TraceParams p) {
     extern __shared__ uint2 sstack[];
     constexpr int LOCAL = kStackTotal - SMEM;
     uint2 lstack[LOCAL];
@@ -160,10 +180,9 @@ __global__ void RQ_KERNEL_BOUNDS cwbvh_kernel(const TraceParams p) {
     Lane L{};
     float ox = 0.f, oy = 0.f, oz = 0.f, dx = 0.f, dy = 0.f, dz = 0.f, tmin = 0.f, tmax = 0.f;
     float idx_ = 0.f, idy = 0.f, idz = 0.f;
-    unsigned octinv = 0, octinv4 = 0;
+    unsigned octinv = 0;
     uint2 ng = make_uint2(0u, 0u), tg = make_uint2(0u, 0u);
-    int sp = 0, hit_addr = -1, steps = 0, nvis = 0, ntri = 0;
-    float hu = 0.f, hv = 0.f;
+    int sp = 0, steps = 0, nvis = 0, ntri = 0;
     bool active = false, exhausted = false;
     const float rt = p.postpone_ratio;
 
@@ -178,27 +197,38 @@ __global__ void RQ_KERNEL_BOUNDS cwbvh_kernel(const TraceParams p) {
         --sp;
         return sp < SMEM ? sstack[(unsigned)sp * B + tid] : lstack[sp - SMEM];
     };
-    auto finish = [&](unsigned err) {
-        if (err) {
-            atomicOr(&p.scratch->error, err);
-            hit_addr = -1;
-        }
-        finish_ray<MULTI>(p, L, tmax, hit_addr, hu, hv);
+    // What only the end of a ray reads waits in shared memory, not in registers.
+    int* const parked = reinterpret_cast<int*>(sstack + (size_t)SMEM * B) + (tid >> 5) * (unsigned)(park_bytes_per_warp(MULTI) / sizeof(int)) + lane;
+    auto woop_limit = [&]() -> unsigned { return MULTI ? (unsigned)parked[224] : p.single.woop_limit; };
+    auto park_hit = [&](int addr, float u, float v) {
+        parked[0] = addr;
+        parked[32] = __float_as_int(u);
+        parked[64] = __float_as_int(v);
+    };
+    auto end_ray = [&](float t, int addr, float u, float v) {
+        const int64_t out = (int64_t)(((uint64_t)(unsigned)parked[128] << 32) | (unsigned)parked[96]);
+        finish_ray<MULTI>(p, MULTI ? parked[160] : 0, out, t, addr, u, v);
         if (COUNT) {
             p.node_visits[L.gidx] = nvis;
             p.tri_tests[L.gidx] = ntri;
         }
         active = false;
     };
+    auto finish = [&](unsigned err) {
+        if (err) atomicOr(&p.scratch->error, err);
+        if (ANY) end_ray(tmax, -1, 0.f, 0.f);
+        else end_ray(tmax, err ? -1 : parked[0], __int_as_float(parked[32]), __int_as_float(parked[64]));
+    };
 
     // Per-warp ray ring after the stacks.
     unsigned char* const ring = reinterpret_cast<unsigned char*>(sstack + (size_t)SMEM * B) +
-                                (size_t)(tid >> 5) * kRingBytesPerWarp;
+                                (size_t)(B >> 5) * park_bytes_per_warp(MULTI) + (size_t)(tid >> 5) * kRingBytesPerWarp;
     float4* const ring_ray = reinterpret_cast<float4*>(ring);
     int64_t* const ring_base = reinterpret_cast<int64_t*>(ring + kRingSlots * sizeof(Ray));
     int* const ring_item = reinterpret_cast<int*>(ring + kRingSlots * sizeof(Ray) + 2 * sizeof(int64_t));
     unsigned cons = 0u;  // next slot to hand out (warp-uniform)
-    int pf_item = -1;  // item of the lane's last prefetched ray (forward search hint)
+    // parked[192]: item of the lane's last prefetched ray (forward search hint)
+    if (RING && MULTI) parked[192] = -1;
     // Takes the next 32 rays from the counter into half `half` of the ring.
     auto claim = [&](unsigned half) {
         unsigned long long base = 0;
@@ -208,8 +238,8 @@ __global__ void RQ_KERNEL_BOUNDS cwbvh_kernel(const TraceParams p) {
         const int64_t g = (int64_t)base + lane;
         if (g < p.total_rays) {
             const unsigned slot = half * kRingHalf + lane;
-            const int item = MULTI ? find_item(p, g, pf_item) : 0;
-            pf_item = item;
+            const int item = MULTI ? find_item(p, g, parked[192]) : 0;
+            if (MULTI) parked[192] = item;
             ring_item[slot] = item;
             const TraceItem* it = MULTI ? p.items + item : &p.single;
             const Ray* src = it->rays + (g - (MULTI ? it->ray_begin : 0));
@@ -229,10 +259,16 @@ __global__ void RQ_KERNEL_BOUNDS cwbvh_kernel(const TraceParams p) {
         idy = guarded_rcp(dy);
         idz = guarded_rcp(dz);
         octinv = 7u - (((dx < 0.f) ? 4u : 0u) | ((dy < 0.f) ? 2u : 0u) | ((dz < 0.f) ? 1u : 0u));
-        octinv4 = octinv * 0x01010101u;
         ng = make_uint2(0u, 0x80000000u);
         tg = make_uint2(0u, 0u);
-        sp = 0; hit_addr = -1; hu = 0.f; hv = 0.f; steps = 0; nvis = 0; ntri = 0;
+        sp = 0; steps = 0; nvis = 0; ntri = 0;
+        if (!ANY) park_hit(-1, 0.f, 0.f);
+        parked[96] = (int)(unsigned)L.out_idx;
+        parked[128] = (int)(unsigned)((uint64_t)L.out_idx >> 32);
+        if (MULTI) {
+            parked[160] = L.item;
+            parked[224] = (int)p.items[L.item].woop_limit;
+        }
         active = true;
     };
 
@@ -297,7 +333,7 @@ __global__ void RQ_KERNEL_BOUNDS cwbvh_kernel(const TraceParams p) {
                 const unsigned slot = (bit - 24u) ^ octinv;
                 const unsigned ci = base + (unsigned)__popc(hitsm & ~(0xFFFFFFFFu << slot));
                 if (++steps > p.step_limit) fault |= kErrTimeout;
-                if (ci >= L.node_limit) fault |= kErrBadScene;
+                if (ci >= (MULTI ? L.node_limit : p.single.node_limit)) fault |= kErrBadScene;
                 if (!fault) {
                     const float4* np = L.nodes + (size_t)ci * 5u;
                     const float4 n0 = ld_nc(np + 0), n1 = ld_nc(np + 1), n2 = ld_nc(np + 2);
@@ -312,7 +348,7 @@ __global__ void RQ_KERNEL_BOUNDS cwbvh_kernel(const TraceParams p) {
                     const float orz = __fmul_rn(-__fsub_rn(oz, n0.z), idz);
                     const bool negx = idx_ < 0.f, negy = idy < 0.f, negz = idz < 0.f;
                     const unsigned hitmask = cwbvh_hitmask<ANY>(n1, n2, n3, n4, adjx, adjy, adjz, orx, ory, orz, negx,
-                                                           negy, negz, octinv4, tmin, tmax);
+                                                           negy, negz, octinv * 0x01010101u, tmin, tmax);
                     ng = make_uint2(__float_as_uint(n1.x), (hitmask & 0xFF000000u) | (ew >> 24));
                     tg = make_uint2(__float_as_uint(n1.y), hitmask & 0x00FFFFFFu);
                 }
@@ -379,7 +415,7 @@ __global__ void RQ_KERNEL_BOUNDS cwbvh_kernel(const TraceParams p) {
                             tri2 = tg.x * 3u + ti2 * 3u;
                             tg.y &= ~(1u << ti2);
                         }
-                        if (tri >= L.woop_limit) {
+                        if (tri >= woop_limit()) {
                             finish(kErrBadScene);
                         } else {
                             const float4* tp = L.woop + tri;
@@ -387,25 +423,27 @@ __global__ void RQ_KERNEL_BOUNDS cwbvh_kernel(const TraceParams p) {
                             float t, u, v;
                             const float4 v0 = ld_nc(tp), v1 = ld_nc(tp + 1), v2 = ld_nc(tp + 2);
                             if (woop_test(v0, v1, v2, ox, oy, oz, dx, dy, dz, tmin, tmax, t, u, v)) {
-                                tmax = t;
-                                hit_addr = (int)tri;
-                                hu = u;
-                                hv = v;
-                                if (ANY) finish(0u);
+                                if (ANY) {
+                                    end_ray(t, (int)tri, u, v);
+                                } else {
+                                    tmax = t;
+                                    park_hit((int)tri, u, v);
+                                }
                             }
                             if (two && active) {
-                                if (tri2 >= L.woop_limit) {
+                                if (tri2 >= woop_limit()) {
                                     finish(kErrBadScene);
                                 } else {
                                     const float4* tp2 = L.woop + tri2;
                                     if (COUNT) ++ntri;
                                     const float4 w0 = ld_nc(tp2), w1 = ld_nc(tp2 + 1), w2 = ld_nc(tp2 + 2);
                                     if (woop_test(w0, w1, w2, ox, oy, oz, dx, dy, dz, tmin, tmax, t, u, v)) {
-                                        tmax = t;
-                                        hit_addr = (int)tri2;
-                                        hu = u;
-                                        hv = v;
-                                        if (ANY) finish(0u);
+                                        if (ANY) {
+                                    end_ray(t, (int)tri2, u, v);
+                                } else {
+                                    tmax = t;
+                                    park_hit((int)tri2, u, v);
+                                }
                                     }
                                 }
                             }
@@ -864,10 +902,10 @@ int lanes_block() { return kLanesBlock; }
 
 int smem_entries_of(int requested) { return requested <= 4 ? 4 : (requested <= 8 ? 8 : 16); }
 
-size_t trace_smem_bytes(rq_bvh_kind kind, int smem_entries, int block, bool ring) {
+size_t trace_smem_bytes(rq_bvh_kind kind, int smem_entries, int block, bool multi, bool ring) {
     if (kind != RQ_BVH_CWBVH) return sizeof(int) * (size_t)smem_entries * (size_t)block;
     return sizeof(uint2) * (size_t)smem_entries * (size_t)block +
-           (ring ? kRingBytesPerWarp * (size_t)(block / 32) : 0);
+           (park_bytes_per_warp(multi) + (ring ? kRingBytesPerWarp : 0)) * (size_t)(block / 32);
 }
 
 }  // namespace rq
