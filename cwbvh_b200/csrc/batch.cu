@@ -367,7 +367,7 @@ rq_status rq_autotune_batch(rq_ctx_t ctx, const rq_batch_item* items, int n_item
     float best_ms = 1e30f;
     rq_batch_params best{};
     const int blocks[] = {64, 128, 256};
-    const int stacks[] = {8, 16};
+    const int stacks[] = {4, 8};  // 16 is never ahead of both (the ring kernels want 4)
     // Sort thresholds: never, items of at least 1M rays, every item.
     const int64_t thresholds[] = {-1, std::min<int64_t>(max_count, 1 << 20), 0};
     rq_status st = RQ_OK;

@@ -77,12 +77,10 @@ struct TraceParams {
 
 typedef void (*TraceKernelFn)(TraceParams);
 
-// ring: the CWBVH any-hit kernel that prefetches rays into a per-warp ring
-// in shared memory (see trace.cu), for batches of at least
-// kRingMinRaysPerThread rays per thread of the grid and single-scene launches
-// of at least kRingMinRaysPerThreadSingle (which have no item search to hide).
-constexpr int64_t kRingMinRaysPerThread = 64;
-constexpr int64_t kRingMinRaysPerThreadSingle = 256;
+// ring: the CWBVH any-hit batch kernel that prefetches rays into a per-warp
+// ring in shared memory (see trace.cu), for batches of at least
+// kRingMinRaysPerThread rays per thread of the grid.
+constexpr int64_t kRingMinRaysPerThread = 16;
 TraceKernelFn trace_kernel(rq_bvh_kind kind, bool any, int smem, bool multi, bool count, bool ring);
 // The CWBVH kernel with g = 8 or 4 lanes to a ray for small launches (see
 // trace.cu), launched with lanes_block() threads per lanes_block() / g rays.

@@ -125,7 +125,7 @@ rq_status launch_trace(rq_bvh_kind kind, rq_query q, const rq_launch& l, bool mu
         }
     }
     RQ_CUDA(cudaMemsetAsync(&p.scratch->ray_counter, 0, sizeof(unsigned long long), s));
-    // Any-hit launches with many rays per thread take the ring-prefetching kernel.
+    // Any-hit batches with many rays per thread take the ring-prefetching kernel.
     TraceParams tp = p;
     TraceKernelFn fn = nullptr;
     size_t smem = 0;
@@ -138,11 +138,9 @@ rq_status launch_trace(rq_bvh_kind kind, rq_query q, const rq_launch& l, bool mu
         if (l.blocks_per_sm > 0) nb = std::min(nb, l.blocks_per_sm);
         tp.fetch_nw = ring && free_shape ? kRingFetchNw : p.fetch_nw;
     };
-    const bool ring = kind == RQ_BVH_CWBVH && !count && q == RQ_ANY;
+    const bool ring = kind == RQ_BVH_CWBVH && !count && multi && q == RQ_ANY;
     pick(ring);
-    if (ring && p.total_rays < (multi ? kRingMinRaysPerThread : kRingMinRaysPerThreadSingle) * device_sms(dev) * nb *
-                                   l.block_size)
-        pick(false);
+    if (ring && p.total_rays < kRingMinRaysPerThread * device_sms(dev) * nb * l.block_size) pick(false);
     int64_t grid = (int64_t)device_sms(dev) * nb;
     // No more warps than rays need.
     const int64_t warps_needed = (p.total_rays + 31) / 32;
@@ -154,7 +152,7 @@ rq_status launch_trace(rq_bvh_kind kind, rq_query q, const rq_launch& l, bool mu
 }
 
 void warm_launch_cache(rq_bvh_kind kind, rq_query q, const rq_launch& l, bool multi, bool count, bool free_shape) {
-    for (int ring = 0; ring <= (kind == RQ_BVH_CWBVH && !count && q == RQ_ANY ? 1 : 0); ++ring) {
+    for (int ring = 0; ring <= (kind == RQ_BVH_CWBVH && !count && multi && q == RQ_ANY ? 1 : 0); ++ring) {
         const int stack = ring && free_shape ? kRingStack : l.smem_stack;
         TraceKernelFn fn = trace_kernel(kind, q == RQ_ANY, stack, multi, count, ring != 0);
         blocks_per_sm(fn, l.block_size, trace_smem_bytes(kind, smem_entries_of(stack), l.block_size, multi, ring != 0));

@@ -42,7 +42,7 @@ constexpr uint32_t kBvh2Sentinel = 0x76543210u;  // src/TraversalKernelBVH2.cu:3
 
 // ------------------------------------------------- per-warp ray prefetch --
 //
-// The CWBVH any-hit kernels of large launches (RING) take rays 32 at a time per
+// The CWBVH any-hit kernel of large batches (RING) takes rays 32 at a time per
 // warp (one counter add per 32 rays) into a ring of 64 slots per warp in
 // shared memory: two halves, each filled by one cp.async group (every lane
 // copies one ray's 32 bytes and notes its batch item).  A refill hands idle
@@ -50,14 +50,13 @@ constexpr uint32_t kBvh2Sentinel = 0x76543210u;  // src/TraversalKernelBVH2.cu:3
 // or more earlier and no longer stall the warp, and neither a counter add nor
 // the item search sits on its path.  A half is refilled as soon as its last
 // slot is handed out.  The last rays of a launch stay tied to the warp whose
-// ring holds them, which costs a short launch more than the ring saves, so
-// the ring is used from kRingMinRaysPerThread rays per thread of the grid up
-// (batches) and from kRingMinRaysPerThreadSingle up (one scene, where no item
-// search is saved): +2 % on a batch of 64 scenes with 127M AO rays, +1 % on
-// 64 scenes with 16.8M rays, +1.6 % on one 29.6M-triangle scene with 64M AO
-// rays (440 per thread), -0.5 % on one scene with 16.8M rays (110 per
-// thread), -6 % on one scene with 1M rays (7 per thread).  Any-hit only:
-// closest-hit batches measured 1 % slower with the ring.
+// ring holds them, which costs a short launch more than the ring saves, so it
+// is used from kRingMinRaysPerThread rays per thread of the grid up.  12 scenes,
+// us without / with the ring: 1.2M rays (7 per thread) 222 / 239, 2.3M (14) 379
+// / 389, 3.9M (23) 645 / 640, 7.9M (46) 1,183 / 1,155.  One scene has no item
+// search to save and loses 1 % even at 64M rays (17,644 / 17,861 on 4M
+// triangles, 11,715 / 11,795 on 100,000).  Any-hit only: closest-hit batches
+// measured 1 % slower with the ring.
 constexpr unsigned kRingHalf = 32;  // rays per counter add
 constexpr unsigned kRingSlots = 2 * kRingHalf;
 // rays [64][2] float4, the two halves' first global ray index, items [64]
@@ -176,7 +175,7 @@ __global__ void RQ_CW_BOUNDS cwbvh_kernel(const TraceParams p) {
     const unsigned tid = threadIdx.x;
     const unsigned B = blockDim.x;
 
-    constexpr bool PAIRS = !(MULTI && RING);
+    static_assert(MULTI || !RING, "the ring is for batches");
     Lane L{};
     float ox = 0.f, oy = 0.f, oz = 0.f, dx = 0.f, dy = 0.f, dz = 0.f, tmin = 0.f, tmax = 0.f;
     float idx_ = 0.f, idy = 0.f, idz = 0.f;
@@ -228,7 +227,7 @@ __global__ void RQ_CW_BOUNDS cwbvh_kernel(const TraceParams p) {
     int* const ring_item = reinterpret_cast<int*>(ring + kRingSlots * sizeof(Ray) + 2 * sizeof(int64_t));
     unsigned cons = 0u;  // next slot to hand out (warp-uniform)
     // parked[192]: item of the lane's last prefetched ray (forward search hint)
-    if (RING && MULTI) parked[192] = -1;
+    if (RING) parked[192] = -1;
     // Takes the next 32 rays from the counter into half `half` of the ring.
     auto claim = [&](unsigned half) {
         unsigned long long base = 0;
@@ -238,11 +237,11 @@ __global__ void RQ_CW_BOUNDS cwbvh_kernel(const TraceParams p) {
         const int64_t g = (int64_t)base + lane;
         if (g < p.total_rays) {
             const unsigned slot = half * kRingHalf + lane;
-            const int item = MULTI ? find_item(p, g, parked[192]) : 0;
-            if (MULTI) parked[192] = item;
+            const int item = find_item(p, g, parked[192]);
+            parked[192] = item;
             ring_item[slot] = item;
-            const TraceItem* it = MULTI ? p.items + item : &p.single;
-            const Ray* src = it->rays + (g - (MULTI ? it->ray_begin : 0));
+            const TraceItem* it = p.items + item;
+            const Ray* src = it->rays + (g - it->ray_begin);
             cp_async16(ring_ray + 2u * slot, &src->origin_tmin);
             cp_async16(ring_ray + 2u * slot + 1u, &src->dir_tmax);
         }
@@ -290,7 +289,7 @@ __global__ void RQ_CW_BOUNDS cwbvh_kernel(const TraceParams p) {
                 const unsigned slot = (cons + rank) & (kRingSlots - 1u);
                 const int64_t g = ring_base[slot / kRingHalf] + (slot & (kRingHalf - 1u));
                 if (g < p.total_rays) {
-                    set_lane<MULTI>(p, g, MULTI ? ring_item[slot] : 0, L);
+                    set_lane<MULTI>(p, g, ring_item[slot], L);
                     Ray r;
                     r.origin_tmin = ring_ray[2u * slot];
                     r.dir_tmax = ring_ray[2u * slot + 1u];
@@ -397,18 +396,16 @@ __global__ void RQ_CW_BOUNDS cwbvh_kernel(const TraceParams p) {
                     }
                     if (want) {
                         // Two triangles of the lane's group per round when it
-                        // has two (PAIRS), in the group's order: the second is
-                        // tested against the tmax the first left, and not at
-                        // all once an any-hit ray has finished (fewer
-                        // warp-wide votes per triangle: +1.0-2.2 % on single
-                        // scenes, +1.3 % on the 64-scene closest-hit batch,
-                        // +2.0 % on a one-item batch; the ring batch kernel
-                        // measured 0.5-1.1 % slower with it on the 64-scene
-                        // AO batch and tests one per round).
+                        // has two, in the group's order: the second is tested
+                        // against the tmax the first left, and not at all once
+                        // an any-hit ray has finished (fewer warp-wide votes
+                        // per triangle: +1.0-2.2 % on single scenes, +1.3 % on
+                        // a 64-scene closest-hit batch, +2.0 % on a one-item
+                        // batch, +-0.2 % in the ring batch kernel).
                         const unsigned ti = highest_bit(tg.y);
                         const unsigned tri = tg.x * 3u + ti * 3u;
                         tg.y &= ~(1u << ti);
-                        const bool two = PAIRS && tg.y != 0u;
+                        const bool two = tg.y != 0u;
                         unsigned tri2 = tri;
                         if (two) {
                             const unsigned ti2 = highest_bit(tg.y);
@@ -876,14 +873,10 @@ static TraceKernelFn select_bvh2(bool any, int smem) {
 TraceKernelFn trace_kernel(rq_bvh_kind kind, bool any, int smem, bool multi, bool count, bool ring) {
     if (kind == RQ_BVH_CWBVH) {
         if (count) return select_cwbvh<false, true, false>(any, smem);
-        if (ring && any) {  // any-hit only (closest-hit batches measured 1 % slower with the ring)
-            if (multi)
-                return smem <= 4 ? (TraceKernelFn)cwbvh_kernel<true, 4, true, false, true>
-                                 : (smem <= 8 ? (TraceKernelFn)cwbvh_kernel<true, 8, true, false, true>
-                                              : (TraceKernelFn)cwbvh_kernel<true, 16, true, false, true>);
-            return smem <= 4 ? (TraceKernelFn)cwbvh_kernel<true, 4, false, false, true>
-                             : (smem <= 8 ? (TraceKernelFn)cwbvh_kernel<true, 8, false, false, true>
-                                          : (TraceKernelFn)cwbvh_kernel<true, 16, false, false, true>);
+        if (ring && any && multi) {
+            return smem <= 4 ? (TraceKernelFn)cwbvh_kernel<true, 4, true, false, true>
+                             : (smem <= 8 ? (TraceKernelFn)cwbvh_kernel<true, 8, true, false, true>
+                                          : (TraceKernelFn)cwbvh_kernel<true, 16, true, false, true>);
         }
         if (!multi) return select_cwbvh<false, false, false>(any, smem);
         return select_cwbvh<true, false, false>(any, smem);
