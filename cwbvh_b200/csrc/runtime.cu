@@ -90,15 +90,17 @@ bool launch_unset(const rq_launch* l) {
 }
 
 // Lanes that share a ray in a CWBVH launch of `rays` rays (0: a lane per ray,
-// the persistent kernel).  Whole calls on 10,592 triangles, us, with
-// 8 lanes / 4 lanes / one, 148 SMs: closest-hit 4,096 rays 24.8 / 29.2 / 50.5,
-// 16,384 30.7 / 33.8 / 53.8, 32,768 49.4 / 39.4 / 55.7, 65,536 85.6 / 69.0 /
-// 62.2; any-hit bakes 4,096 30.5 / 32.8 / 53.4, 16,384 35.8 / 37.9 / 61.1,
-// 65,536 67.6 / 59.5 / 66.9, 262,144 230 / 183 / 128.  (Two lanes to a ray are
+// the persistent kernel), on 148 SMs.  8 and 4 lanes cross at 128 rays per SM
+// (whole calls on 10,592 triangles, us, 8 / 4 lanes: closest-hit 4,096 rays
+// 24.8 / 29.2, 16,384 30.7 / 33.8, 32,768 49.4 / 39.4).  4 lanes and one cross
+// later the deeper the scene: closest-hit, 4 / one, 65,536 rays on 3,000 / 10,592
+// / 60,000 / 200,000 triangles 40 / 39.5, 59 / 62, 85 / 92, 120 / 143 us, 75,000
+// 43 / 40, 64 / 64, 92 / 94, 125 / 145; any-hit 75,000 38 / 39, 52 / 54, 60 / 74,
+// 64 / 72, 85,000 42 / 41, 55 / 57, 67 / 75, 71 / 73.  (Two lanes to a ray are
 // never the fastest.)
 static int lanes_per_ray(rq_query q, int64_t rays, int sms) {
     if (rays <= 128 * (int64_t)sms) return 8;
-    return rays <= (q == RQ_ANY ? 448 : 320) * (int64_t)sms ? 4 : 0;
+    return rays <= (q == RQ_ANY ? 520 : 440) * (int64_t)sms ? 4 : 0;
 }
 
 // Stack entries per lane in shared memory of the ring kernels where the caller
