@@ -78,14 +78,15 @@ __device__ __forceinline__ void cwbvh_visit(const float4* np, float ox, float oy
 // the city of 625 instances, 4.2M primary rays closest-hit / one AO ray each
 // any-hit, us: 1,394 / 836 as it was; 1,362 / 806 with the world ray kept in
 // shared memory instead of read and inverted again on leaving an instance;
-// 1,294 / 798 with pairs of triangle tests as in the flat kernel and 72
-// registers, seven blocks per SM (64 and eight: 1,303 / 814; 80 and six: 1,353
-// / 841; 56 and nine spill: 1,411 / 845); 1,131 / 786 with refills at Nd 6 / Nw
-// 32 instead of 2 / 8 (4 / 16: 1,183 / 792), which keep a warp's camera rays
-// together; 1,115 / 777 with 32-bit limits and branch-free triangle
-// acceptance.  Entering instances only when 4 or 8 lanes would: 3-6 % slower.
+// 1,294 / 798 with pairs of triangle tests as in the flat kernel; 1,131 / 786
+// with refills at Nd 6 / Nw 32 instead of 2 / 8 (4 / 16: 1,183 / 792), which
+// keep a warp's camera rays together; 1,115 / 777 with 32-bit limits and
+// branch-free triangle acceptance; 1,102 / 746 with the hit and the ray index
+// parked in shared memory, which lets 64 registers do, eight blocks per SM (72
+// and seven: 1,112 / 774; 56 and nine spill: 1,174 / 781).  Entering instances
+// only when 4 or 8 lanes would: 3-6 % slower.
 template <bool ANY, int SMEM>
-__global__ void __launch_bounds__(128, 7) cwbvh_inst_kernel(const InstParams p) {
+__global__ void __launch_bounds__(128, 8) cwbvh_inst_kernel(const InstParams p) {
     extern __shared__ uint2 sstack[];
     constexpr int LOCAL = kInstStack - SMEM;
     uint2 lstack[LOCAL];
@@ -102,11 +103,9 @@ __global__ void __launch_bounds__(128, 7) cwbvh_inst_kernel(const InstParams p) 
 
     float ox = 0.f, oy = 0.f, oz = 0.f, dx = 0.f, dy = 0.f, dz = 0.f, tmin = 0.f, tmax = 0.f;
     float idx_ = 0.f, idy = 0.f, idz = 0.f;
-    unsigned octinv = 0, octinv4 = 0;
+    unsigned octinv = 0;
     uint2 ng = make_uint2(0u, 0u), tg = make_uint2(0u, 0u);
-    int sp = 0, hit_addr = -1, hit_inst = -1, steps = 0;
-    int64_t ray = 0;
-    float hu = 0.f, hv = 0.f;
+    int sp = 0, steps = 0;
     bool active = false, exhausted = false;
 
     auto push = [&](uint2 v) -> bool {
@@ -122,7 +121,6 @@ __global__ void __launch_bounds__(128, 7) cwbvh_inst_kernel(const InstParams p) 
     };
     auto set_octant = [&]() {
         octinv = 7u - (((dx < 0.f) ? 4u : 0u) | ((dy < 0.f) ? 2u : 0u) | ((dz < 0.f) ? 1u : 0u));
-        octinv4 = octinv * 0x01010101u;
     };
     auto set_ray = [&](float4 o, float4 d) {
         ox = o.x; oy = o.y; oz = o.z;
@@ -134,6 +132,9 @@ __global__ void __launch_bounds__(128, 7) cwbvh_inst_kernel(const InstParams p) 
     };
     // The world ray, nine words per lane after the stacks.
     float* const world = reinterpret_cast<float*>(sstack + SMEM * B) + tid;
+    // What only the end of a ray reads, in the six words after that: hit
+    // address, instance, u, v and the ray index in two halves.
+    int* const parked = reinterpret_cast<int*>(sstack + SMEM * B) + 9 * B + tid;
     auto top_level = [&]() {
         in_blas = false;
         nodes = p.tlas_nodes; woop = p.tlas_rows; node_limit = p.tlas_node_limit; woop_limit = p.tlas_rows_limit;
@@ -145,15 +146,23 @@ __global__ void __launch_bounds__(128, 7) cwbvh_inst_kernel(const InstParams p) 
         idx_ = world[6 * B]; idy = world[7 * B]; idz = world[8 * B];
         set_octant();
     };
-    auto finish = [&](unsigned err) {
-        if (err) {
-            atomicOr(&p.scratch->error, err);
-            hit_addr = -1;
-            hit_inst = -1;
-        }
-        __stcs(&p.hits[ray].t_triId_u_v, make_float4(tmax, __int_as_float(hit_addr), hu, hv));
-        if (p.inst_out) p.inst_out[ray] = hit_addr >= 0 ? hit_inst : -1;
+    auto end_ray = [&](float t, int addr, int inst, float u, float v) {
+        const int64_t ray = (int64_t)(((uint64_t)(unsigned)parked[5 * B] << 32) | (unsigned)parked[4 * B]);
+        __stcs(&p.hits[ray].t_triId_u_v, make_float4(t, __int_as_float(addr), u, v));
+        if (p.inst_out) p.inst_out[ray] = addr >= 0 ? inst : -1;
         active = false;
+    };
+    auto finish = [&](unsigned err) {
+        if (err) atomicOr(&p.scratch->error, err);
+        if (ANY) end_ray(tmax, -1, -1, 0.f, 0.f);
+        else end_ray(tmax, err ? -1 : parked[0], parked[B], __int_as_float(parked[2 * B]),
+                     __int_as_float(parked[3 * B]));
+    };
+    auto park_hit = [&](int addr, int inst, float u, float v) {
+        parked[0] = addr;
+        parked[B] = inst;
+        parked[2 * B] = __float_as_int(u);
+        parked[3 * B] = __float_as_int(v);
     };
 
     for (;;) {
@@ -167,7 +176,8 @@ __global__ void __launch_bounds__(128, 7) cwbvh_inst_kernel(const InstParams p) 
             if (need) {
                 const int64_t g = (int64_t)base + __popc(needm & lanemask_lt());
                 if (g < p.total_rays) {
-                    ray = g;
+                    parked[4 * B] = (int)(unsigned)g;
+                    parked[5 * B] = (int)(unsigned)((uint64_t)g >> 32);
                     const float4 o = __ldg(&p.rays[g].origin_tmin), d = __ldg(&p.rays[g].dir_tmax);
                     top_level();
                     set_ray(o, d);
@@ -179,7 +189,8 @@ __global__ void __launch_bounds__(128, 7) cwbvh_inst_kernel(const InstParams p) 
                     ng = make_uint2(0u, 0x80000000u);
                     tg = make_uint2(0u, 0u);
                     sp = 0; inst_sp = 0; cur_inst = -1;
-                    hit_addr = -1; hit_inst = -1; hu = 0.f; hv = 0.f; steps = 0;
+                    steps = 0;
+                    if (!ANY) park_hit(-1, -1, 0.f, 0.f);
                     active = true;
                 } else {
                     exhausted = true;
@@ -203,8 +214,8 @@ __global__ void __launch_bounds__(128, 7) cwbvh_inst_kernel(const InstParams p) 
                     const unsigned ci = base + (unsigned)__popc(hitsm & ~(0xFFFFFFFFu << slot));
                     if (++steps > p.step_limit) fault |= kErrTimeout;
                     if (ci >= node_limit) fault |= kErrBadScene;
-                    if (!fault) cwbvh_visit(nodes + (size_t)ci * 5u, ox, oy, oz, idx_, idy, idz, octinv4, tmin, tmax,
-                                            ng, tg);
+                    if (!fault) cwbvh_visit(nodes + (size_t)ci * 5u, ox, oy, oz, idx_, idy, idz, octinv * 0x01010101u,
+                                            tmin, tmax, ng, tg);
                 } else {
                     tg = ng;
                     ng = make_uint2(0u, 0u);
@@ -238,12 +249,12 @@ __global__ void __launch_bounds__(128, 7) cwbvh_inst_kernel(const InstParams p) 
                         auto test = [&](const float4& a, const float4& b, const float4& c, unsigned addr) {
                             float t, u, v;
                             if (woop_test(a, b, c, ox, oy, oz, dx, dy, dz, tmin, tmax, t, u, v)) {
-                                tmax = t;
-                                hit_addr = (int)addr;
-                                hit_inst = cur_inst;
-                                hu = u;
-                                hv = v;
-                                if (ANY) finish(0u);
+                                if (ANY) {
+                                    end_ray(t, (int)addr, cur_inst, u, v);
+                                } else {
+                                    tmax = t;
+                                    park_hit((int)addr, cur_inst, u, v);
+                                }
                             }
                         };
                         test(r0, r1, r2, tri);
@@ -412,7 +423,8 @@ rq_status rq_trace_instanced(rq_ctx_t ctx, rq_tlas_t tlas, const rq_ray* rays, r
     p.step_limit = l.step_limit;
     constexpr int kSmem = 8, kBlock = 128;
     void (*fn)(InstParams) = query == RQ_ANY ? cwbvh_inst_kernel<true, kSmem> : cwbvh_inst_kernel<false, kSmem>;
-    const size_t smem = (kSmem * sizeof(uint2) + 9 * sizeof(float)) * (size_t)kBlock;  // stacks, world rays
+    // per lane: the stack, nine words of the world ray, six that only its end reads
+    const size_t smem = (kSmem * sizeof(uint2) + (9 + 6) * sizeof(float)) * (size_t)kBlock;
     int per_sm = 0;
     RQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kBlock, smem));
     const int64_t blocks_needed = (count + kBlock - 1) / kBlock;

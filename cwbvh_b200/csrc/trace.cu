@@ -68,9 +68,9 @@ static_assert(kRingBytesPerWarp % 16 == 0, "ring keeps 16 B alignment");
 // and for a batch its item, the prefetched item and the item's Woop limit.  With
 // them in registers the kernels took 64 and eight 128-thread blocks fit an SM;
 // without, 56 and nine, with no spills (10 B in the ring batch kernel with more
-// than four stack entries; 72 registers and seven blocks are 1-6 % slower than 64, 48 and ten spill and
-// are 2-10 % slower).  Single-scene kernels read the limits from the launch
-// parameters.  4.2M city primary rays 808 -> 795 us, 4M AO rays on 4M triangles
+// than four stack entries; 72 registers and seven blocks are 1-6 % slower than
+// 64, 48 and ten spill and are 2-10 % slower).  Single-scene kernels read the
+// limits from the launch parameters.  4.2M city primary rays 808 -> 795 us, 4M AO rays on 4M triangles
 // 1,240 -> 1,204 us, 1M closest hits 390 -> 389 us, 18M AO rays of 12 scenes
 // 3,332 -> 3,205 us (with four stack entries, see launch_trace).
 constexpr int kParkWordsSingle = 5, kParkWordsMulti = 8;
