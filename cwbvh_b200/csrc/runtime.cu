@@ -93,14 +93,16 @@ bool launch_unset(const rq_launch* l) {
 // the persistent kernel), on 148 SMs.  8 and 4 lanes cross at 128 rays per SM
 // (whole calls on 10,592 triangles, us, 8 / 4 lanes: closest-hit 4,096 rays
 // 24.8 / 29.2, 16,384 30.7 / 33.8, 32,768 49.4 / 39.4).  4 lanes and one cross
-// later the deeper the scene: closest-hit, 4 / one, 65,536 rays on 3,000 / 10,592
-// / 60,000 / 200,000 triangles 40 / 39.5, 59 / 62, 85 / 92, 120 / 143 us, 75,000
-// 43 / 40, 64 / 64, 92 / 94, 125 / 145; any-hit 75,000 38 / 39, 52 / 54, 60 / 74,
-// 64 / 72, 85,000 42 / 41, 55 / 57, 67 / 75, 71 / 73.  (Two lanes to a ray are
-// never the fastest.)
-static int lanes_per_ray(rq_query q, int64_t rays, int sms) {
+// at 270-500 rays per SM, sooner where neighbouring rays go different ways and
+// the scene is shallow.  4 lanes / one, us, 32,000 / 40,000 / 49,000 / 65,000
+// rays: any-hit, one ray per surfel, city of 120,000 triangles 31/39, 42/40,
+// 44/41, 50/43, heightfield of 60,000 39/52, 48/53, 55/54, 65/56; 32 per surfel
+// 31/41, 35/41, 40/42, 46/43 and 39/56, 41/63, 48/63, 57/64; closest-hit, one per
+// surfel 39/51, 52/51, 57/52, 66/54 and 54/71, 72/73, 83/77, 94/80.  (Two lanes
+// to a ray are never the fastest.)
+static int lanes_per_ray(int64_t rays, int sms) {
     if (rays <= 128 * (int64_t)sms) return 8;
-    return rays <= (q == RQ_ANY ? 520 : 440) * (int64_t)sms ? 4 : 0;
+    return rays <= 270 * (int64_t)sms ? 4 : 0;
 }
 
 // Stack entries per lane in shared memory of the ring kernels where the caller
@@ -117,7 +119,7 @@ rq_status launch_trace(rq_bvh_kind kind, rq_query q, const rq_launch& l, bool mu
     int dev = 0;
     RQ_CUDA(cudaGetDevice(&dev));
     if (free_shape && kind == RQ_BVH_CWBVH && !count) {
-        if (const int g = lanes_per_ray(q, p.total_rays, device_sms(dev))) {
+        if (const int g = lanes_per_ray(p.total_rays, device_sms(dev))) {
             const int64_t rays_per_block = lanes_block() / g;
             const unsigned blocks = (unsigned)((p.total_rays + rays_per_block - 1) / rays_per_block);
             void* args[] = {(void*)&p};

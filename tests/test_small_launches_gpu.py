@@ -15,20 +15,18 @@ def scene(rq):
     V, I = W.heightfield_boxes(5)
     ds = W.upload(V, I, rq.CWBVH)
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    rays = W.ao_rays(ds, 520 * sms, seed=31, tmax_scale=1.0).cpu().numpy()
+    rays = W.ao_rays(ds, 270 * sms, seed=31, tmax_scale=1.0).cpu().numpy()
     rays[::5, 3] = 0.0      # tmin = 0 and < 0 beside ordinary rays
     rays[1::7, 3] = -0.25
     return ds, rays, sms
 
 
 @pytest.mark.parametrize("query", [0, 1], ids=["closest", "any"])
-@pytest.mark.parametrize("n", [1, 15, 16, 17, 33, 4096, (128, 0), (128, 1), (320, 0), (440, 0), (520, 0)], ids=str)
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 33, 4096, (128, 0), (128, 1), (270, 0)], ids=str)
 def test_small_launch_bit_exact(rq, po, scene, n, query):
     import torch
     ds, rays, sms = scene
     n = n if isinstance(n, int) else n[0] * sms + n[1]
-    if query == rq.CLOSEST:
-        n = min(n, 440 * sms)
     r = np.ascontiguousarray(rays[:n])
     hits = torch.full((n + 8, 4), 5.0, device="cuda")
     ctx = rq.Context()
