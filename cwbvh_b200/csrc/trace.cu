@@ -9,10 +9,11 @@
 // src/TraversalKernelCWBVH.cu:56-87, written with __shfl_sync instead of a
 // volatile shared word so it is correct under independent thread scheduling).
 // A warp re-fills after the idle lanes have cost Nw lane-iterations beyond Nd
-// (src/TraversalKernelCWBVH.cu:365-371).  Large CWBVH any-hit launches take
-// their rays through a per-warp ring of prefetched rays instead (below).  Every vote is
-// over the full warp and every loop is warp-uniform, so lanes never diverge
-// around a collective.
+// (src/TraversalKernelCWBVH.cu:365-371).  Large CWBVH any-hit batches take
+// their rays through a per-warp ring of prefetched rays instead (below), and
+// the last rays of a CWBVH launch get four lanes each.  Every vote is over the
+// full warp and every loop is warp-uniform, so lanes never diverge around a
+// collective.
 //
 // Safety.  A ray whose stack would overflow, whose node/triangle index falls
 // outside the buffers, or that runs more than the step limit is finished as
@@ -508,7 +509,7 @@ __global__ void RQ_CW_BOUNDS cwbvh_kernel(const TraceParams p) {
         // that far).  us before / after: AO 94k, 262k, 524k rays on 200,000
         // triangles 74 / 67, 117 / 104, 165 / 149, closest-hit 149 / 136, 222 /
         // 201, 341 / 315; 1M AO rays on 10,592 215 / 204, 1M closest-hit on
-        // 200,000 388 / 372, 4M AO rays on 4M 1,202 / 1,178, batches of 1.2M
+        // 20,000 388 / 372, 4M AO rays on 4M 1,202 / 1,178, batches of 1.2M
         // and 7.9M rays 220 / 208, 1,151 / 1,145.  Eight lanes from 4 rays on
         // gain 60-75 % of that, two from 16 on 50-75 %.
         if (!COUNT && __any_sync(kFullMask, exhausted) && __popc(live) <= kTailRays &&
