@@ -1271,6 +1271,15 @@ __global__ void __launch_bounds__(kExpandBlock) expand_kernel(
             }
             if (!__any_sync(kWarpAll, who < 64)) break;
         }
+        // Costs that are not below FLT_MAX (infinite or NaN vertices, centres
+        // that overflow) choose nothing: those children take the free slots in
+        // order, since every inner child's place in the queue will be read.
+        const unsigned unplaced = octet(has && my_slot < 0);
+        if (has && my_slot < 0) {
+            unsigned f = free_slots;
+            for (int rank = __popc(unplaced & ((1u << c) - 1u)); rank > 0; --rank) f &= f - 1u;
+            my_slot = __ffs(f) - 1;
+        }
         // ---- per-axis exponent, grown while a child's upper bound does not fit a byte
         int e[3];
         for (int a = 0; a < 3; ++a) {
@@ -1306,10 +1315,9 @@ __global__ void __launch_bounds__(kExpandBlock) expand_kernel(
         err = all_or(err);  // of the group
         const bool go = active && err == 0u;
         // ---- the node
-        const bool placed = has && my_slot >= 0;
-        const unsigned imask = all_or(placed && inner ? 1u << my_slot : 0u);
-        const unsigned counts = all_or(placed && leaf ? (unsigned)b.count << (2 * my_slot) : 0u);
-        const unsigned below = placed ? counts & ((1u << (2 * my_slot)) - 1u) : 0u;
+        const unsigned imask = all_or(inner ? 1u << my_slot : 0u);
+        const unsigned counts = all_or(leaf ? (unsigned)b.count << (2 * my_slot) : 0u);
+        const unsigned below = has ? counts & ((1u << (2 * my_slot)) - 1u) : 0u;
         const unsigned first_tri = __popc(below & 0x5555u) + 2u * __popc(below & 0xAAAAu);
         const unsigned all_tris = __popc(counts & 0x5555u) + 2u * __popc(counts & 0xAAAAu);
         if (c < 5) node_smem[group][c] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1321,7 +1329,7 @@ __global__ void __launch_bounds__(kExpandBlock) expand_kernel(
                                                               (((unsigned)e[2] & 0xFFu) << 16) | (imask << 24)));
             reinterpret_cast<uint2*>(bytes)[2] = make_uint2(imask ? base : 0u, all_tris ? tbase : 0u);
         }
-        if (go && placed) {
+        if (go && has) {
             for (int a = 0; a < 3; ++a) {
                 const float scale = ldexpf(1.0f, e[a]);
                 bytes[32 + my_slot + 8 * a] = (uint8_t)(int)floorf((b.lo[a] - lo[a]) / scale);
