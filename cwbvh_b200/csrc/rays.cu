@@ -596,13 +596,15 @@ rq_status rq_sort_rays(rq_ctx_t ctx, const rq_ray* rays, int64_t count, const fl
     if (count == 0) return RQ_OK;
     cudaStream_t s = (cudaStream_t)stream;
     const size_t n = (size_t)count;
-    // Outputs that overlap the input or each other are written last, from copies.
+    // Outputs that overlap the input or each other, or that the kernels' stores
+    // are too wide for (rays 16 bytes, numbers 4), are written last, from copies.
     auto overlap = [](const void* a, size_t an, const void* b, size_t bn) {
         return (uintptr_t)a < (uintptr_t)b + bn && (uintptr_t)b < (uintptr_t)a + an;
     };
     const bool staged = overlap(rays, n * sizeof(Ray), sorted_rays, n * sizeof(Ray)) ||
                         overlap(rays, n * sizeof(Ray), perm, n * 4) ||
-                        overlap(sorted_rays, n * sizeof(Ray), perm, n * 4);
+                        overlap(sorted_rays, n * sizeof(Ray), perm, n * 4) ||
+                        ((uintptr_t)sorted_rays & 15u) != 0 || ((uintptr_t)perm & 3u) != 0;
     size_t cub_bytes = 0;
     RQ_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, cub_bytes, (const uint32_t*)nullptr, (uint32_t*)nullptr,
                                             (const int32_t*)nullptr, (int32_t*)nullptr, count, 0, kRayKeyBits, s));

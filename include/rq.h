@@ -306,7 +306,7 @@ rq_status rq_ao_reduce(const rq_hit* hits, int64_t n_surfels, int spp, float* ou
  * the permutation (sorted position -> original index); waits for the stream.
  * Sort buffers of up to 256 MB (about 20M rays) stay with the context until
  * it is destroyed; larger ones are allocated and freed by the call.  Outputs
- * may overlap the input or each other. */
+ * may overlap the input or each other and lie at any address. */
 rq_status rq_sort_rays(rq_ctx_t ctx, const rq_ray* rays, int64_t count, const float bounds_lo[3],
                        const float bounds_hi[3], rq_ray* sorted_rays, int32_t* perm,
                        void* stream);
