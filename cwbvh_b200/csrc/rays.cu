@@ -262,11 +262,12 @@ __global__ void surfels_from_hits_kernel(const Ray* __restrict__ rays, const Hit
 template <int P>
 __global__ void ao_reduce_kernel(const Hit* __restrict__ hits, int64_t n_surfels, int spp, float* __restrict__ ao) {
     const int64_t s = (int64_t)blockIdx.x * (blockDim.x / P) + threadIdx.x / P;
-    const int c = (int)(threadIdx.x % P);
+    const unsigned c = threadIdx.x % P, n = (unsigned)spp;
     int occ = 0;
     if (s < n_surfels)
 #pragma unroll 4
-        for (int k = c; k < spp; k += P) occ += __float_as_int(hits[s * spp + k].t_triId_u_v.y) != -1;
+        for (unsigned k = c; k < n; k += P)  // unsigned: k ends up to P - 1 past spp, which may be past INT_MAX
+            occ += __float_as_int(hits[s * spp + k].t_triId_u_v.y) != -1;
 #pragma unroll
     for (int m = P / 2; m > 0; m >>= 1) occ += __shfl_xor_sync(kFullMask, occ, m);
     if (c == 0 && s < n_surfels) ao[s] = (float)occ / (float)spp;
