@@ -1926,7 +1926,10 @@ extern "C" rq_status rq_build_scene_gpu(const float* vertices, int64_t nv, const
     }
     const rq_status st = build_scene(vertices, nv, indices, nt, method | (thread_treelets ? RQ_GPU_BUILD_THREAD_TREELETS : 0),
                                      optimize_passes, split_budget, out, pool, device, (cudaStream_t)stream);
-    if (st != RQ_OK) scratch_pool().leave(device);  // otherwise the scene does, when it is destroyed
+    if (st != RQ_OK) {  // otherwise the scene leaves, when it is destroyed
+        cudaStreamSynchronize((cudaStream_t)stream);  // the frees queued on it are done
+        scratch_pool().leave(device);
+    }
     return st;
 }
 
@@ -2094,6 +2097,10 @@ static rq_status build_scene(const float* vertices, int64_t nv, const int32_t* i
     float root[20] = {};
     if (st == RQ_OK)
         ok(cudaMemcpyAsync(root, nodes, sizeof(root), cudaMemcpyDeviceToHost, s), "rq_build_scene_gpu");
+    // Freed before the host's last wait: the pool gives back, with the last
+    // scene, only what it has seen the stream let go of.
+    arena.release();
+    rm.arena.release();
     ok(cudaStreamSynchronize(s), "rq_build_scene_gpu");
     if (st != RQ_OK) {
         cudaFree(block);
