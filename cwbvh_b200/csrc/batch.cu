@@ -17,7 +17,6 @@ struct rq_batch {
     rq_query query = RQ_ANY;
     rq_bvh_kind kind = RQ_BVH_CWBVH;
     rq_launch launch{};
-    bool free_shape = false;  // no launch shape was asked for
     rq_batch_params params{};
     std::vector<rq::TraceItem> items;  // host copy (ray_begin = global prefix)
     rq::TraceItem* d_items = nullptr;
@@ -40,7 +39,7 @@ static rq_status batch_enqueue(rq_batch* b, cudaStream_t s) {
     p.items = b->d_items;
     p.n_items = (int)b->items.size();
     p.total_rays = b->total;
-    return launch_trace(b->kind, b->query, b->launch, true, false, b->free_shape, p, s);
+    return launch_trace(b->kind, b->query, b->launch, true, false, p, s);
 }
 
 }  // namespace rq
@@ -67,7 +66,6 @@ rq_status rq_batch_create(rq_ctx_t ctx, const rq_batch_item* items, int n_items,
     if (params) b->params = *params;
     else b->params.sort_threshold = -1;
     b->launch = resolve_launch(kind, query, params ? &params->launch : nullptr);
-    b->free_shape = launch_unset(params ? &params->launch : nullptr);
 
     std::vector<TraceItem> to_sort;
     std::vector<float> bounds;
@@ -119,7 +117,7 @@ rq_status rq_batch_run(rq_batch_t b, void* stream) {
     cudaStream_t s = (cudaStream_t)stream;
     if (!b->params.use_graph || s == nullptr) return batch_enqueue(b, s);
     if (!b->exec) {
-        warm_launch_cache(b->kind, b->query, b->launch, true, false, b->free_shape);
+        warm_launch_cache(b->kind, b->query, b->launch, true, false);
         RQ_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeRelaxed));
         rq_status st = batch_enqueue(b, s);
         cudaGraph_t g = nullptr;
@@ -145,7 +143,7 @@ rq_status rq_batch_run_stage(rq_batch_t b, int stage, void* stream) {
     p.items = b->d_items;
     p.n_items = (int)b->items.size();
     p.total_rays = b->total;
-    return launch_trace(b->kind, b->query, b->launch, true, false, b->free_shape, p, s);
+    return launch_trace(b->kind, b->query, b->launch, true, false, p, s);
 }
 
 int rq_batch_kernel_count(rq_batch_t b) {
@@ -188,6 +186,10 @@ namespace rq {
 
 static std::mutex g_tune_mu;
 
+// Part of the cache key: raised when the kernels change enough to change which
+// shapes are the fastest, so that choices timed on earlier ones are made again.
+constexpr const char* kTuneRevision = "r2";
+
 static std::string tune_key(rq_bvh_kind kind, rq_query q, int64_t count) {
     int dev = 0;
     cudaGetDevice(&dev);
@@ -200,7 +202,7 @@ static std::string tune_key(rq_bvh_kind kind, rq_query q, int64_t count) {
         if (c == ' ') c = '_';
     std::ostringstream os;
     os << name << "|" << (kind == RQ_BVH_CWBVH ? "cwbvh" : "bvh2") << "|" << (q == RQ_ANY ? "any" : "closest") << "|"
-       << cls;
+       << cls << "|" << kTuneRevision;
     return os.str();
 }
 
@@ -367,7 +369,11 @@ rq_status rq_autotune_batch(rq_ctx_t ctx, const rq_batch_item* items, int n_item
     float best_ms = 1e30f;
     rq_batch_params best{};
     const int blocks[] = {64, 128, 256};
-    const int stacks[] = {4, 8};  // 16 is never ahead of both (the ring kernels want 4)
+    // The ring kernels want 4 entries (12 x 800,000 AO rays, 128 threads, 4 / 8
+    // / 16: 1,806 / 1,872 / 2,036 us), the others 8 (closest-hit batches 3,537 /
+    // 3,504 / 3,515, BVH2 3,289 / 3,216 / 3,219, BVH2 any-hit 2,248 / 2,189 /
+    // 2,188); 16 is nowhere more than 0.3 % ahead of both.
+    const int stacks[] = {4, 8};
     // Sort thresholds: never, items of at least 1M rays, every item.
     const int64_t thresholds[] = {-1, std::min<int64_t>(max_count, 1 << 20), 0};
     rq_status st = RQ_OK;

@@ -84,9 +84,14 @@ static int blocks_per_sm(TraceKernelFn fn, int block, size_t smem) {
     return cache[key];
 }
 
-bool launch_unset(const rq_launch* l) {
-    return !l || (l->block_size == 0 && l->blocks_per_sm == 0 && l->smem_stack == 0 && l->postpone_ratio == 0.f &&
-                  l->fetch_nd == 0 && l->fetch_nw == 0);
+// Whether a resolved launch is the default one in all that shapes the kernel,
+// so that the library may choose another kernel or stack size.  It counts as
+// that however it was asked for: by zeros, by the values that
+// rq_default_launch returns, or by a tuner that found them the fastest.
+static bool default_shape(rq_bvh_kind kind, rq_query q, const rq_launch& l) {
+    const rq_launch d = resolve_launch(kind, q, nullptr);
+    return l.block_size == d.block_size && l.blocks_per_sm == d.blocks_per_sm && l.smem_stack == d.smem_stack &&
+           l.postpone_ratio == d.postpone_ratio && l.fetch_nd == d.fetch_nd && l.fetch_nw == d.fetch_nw;
 }
 
 // Lanes that share a ray in a CWBVH launch of `rays` rays (0: a lane per ray,
@@ -105,17 +110,18 @@ static int lanes_per_ray(int64_t rays, int sms) {
     return rays <= 270 * (int64_t)sms ? 4 : 0;
 }
 
-// Stack entries per lane in shared memory of the ring kernels where the caller
-// leaves the shape open: nine blocks with rings and eight entries leave L1 28 KB
+// Stack entries per lane in shared memory of the ring kernels where the shape is
+// the default one: nine blocks with rings and eight entries leave L1 28 KB
 // (18M AO rays of 12 scenes 3,370 us), with four 60 KB (3,205 us).  The kernels
 // without rings are the same within 1 % from 4 to 16.  A refill from the ring
 // is cheap, so they also refill sooner, at Nw 4 instead of 8 (3,178 us; the
 // others lose 1 % by it).
 constexpr int kRingStack = 4, kRingFetchNw = 4;
 
-rq_status launch_trace(rq_bvh_kind kind, rq_query q, const rq_launch& l, bool multi, bool count, bool free_shape,
+rq_status launch_trace(rq_bvh_kind kind, rq_query q, const rq_launch& l, bool multi, bool count,
                        const TraceParams& p, cudaStream_t s) {
     if (p.total_rays <= 0) return RQ_OK;
+    const bool free_shape = default_shape(kind, q, l);
     int dev = 0;
     RQ_CUDA(cudaGetDevice(&dev));
     if (free_shape && kind == RQ_BVH_CWBVH && !count) {
@@ -155,7 +161,8 @@ rq_status launch_trace(rq_bvh_kind kind, rq_query q, const rq_launch& l, bool mu
     return RQ_OK;
 }
 
-void warm_launch_cache(rq_bvh_kind kind, rq_query q, const rq_launch& l, bool multi, bool count, bool free_shape) {
+void warm_launch_cache(rq_bvh_kind kind, rq_query q, const rq_launch& l, bool multi, bool count) {
+    const bool free_shape = default_shape(kind, q, l);
     for (int ring = 0; ring <= (kind == RQ_BVH_CWBVH && !count && multi && q == RQ_ANY ? 1 : 0); ++ring) {
         const int stack = ring && free_shape ? kRingStack : l.smem_stack;
         TraceKernelFn fn = trace_kernel(kind, q == RQ_ANY, stack, multi, count, ring != 0);
@@ -413,7 +420,7 @@ static rq_status trace_impl(rq_ctx_t ctx, rq_scene_t scene, const rq_ray* rays, 
     p.single.ao_counts = ao_counts;
     p.single.ao_spp = ao_spp;
     if (speculative >= 0) p.bvh2_speculative = speculative;
-    return launch_trace(scene->kind, query, l, false, nv != nullptr, launch_unset(launch), p, (cudaStream_t)stream);
+    return launch_trace(scene->kind, query, l, false, nv != nullptr, p, (cudaStream_t)stream);
 }
 
 rq_status rq_trace(rq_ctx_t ctx, rq_scene_t scene, const rq_ray* rays, rq_hit* hits, int64_t count, rq_query query,

@@ -52,17 +52,14 @@ void gpu_built_scene_gone(int device);
 // Fills zero fields of `l` with defaults for this BVH kind / query.
 rq_launch resolve_launch(rq_bvh_kind kind, rq_query q, const rq_launch* l);
 
-// Whether a caller's launch leaves the kernel's shape to the library.
-bool launch_unset(const rq_launch* l);
-
 // Launches the trace kernel for p's rays (and zeroes the ray counter for the
-// persistent ones).  `free_shape`: the caller named no launch shape, so small
-// CWBVH launches may take the kernel with several lanes to a ray.
-rq_status launch_trace(rq_bvh_kind kind, rq_query q, const rq_launch& l, bool multi, bool count, bool free_shape,
+// persistent ones).  With the default launch shape, small CWBVH launches take
+// the kernel with several lanes to a ray.
+rq_status launch_trace(rq_bvh_kind kind, rq_query q, const rq_launch& l, bool multi, bool count,
                        const TraceParams& p, cudaStream_t s);
 
 // Computes the occupancy of a kernel variant ahead of a stream capture.
-void warm_launch_cache(rq_bvh_kind kind, rq_query q, const rq_launch& l, bool multi, bool count, bool free_shape);
+void warm_launch_cache(rq_bvh_kind kind, rq_query q, const rq_launch& l, bool multi, bool count);
 
 // Zeroes the context's ray counter on the stream.
 rq_status reset_counter(rq_ctx* ctx, cudaStream_t s);

@@ -331,7 +331,7 @@ void rq_server::launch_batch(Worker& w, std::vector<Piece*>& batch, int32_t batc
         p.items = reinterpret_cast<const rq::TraceItem*>(w.d_table);
         p.n_items = (int)batch.size();
         p.total_rays = ray_begin;
-        st = rq::launch_trace(kind, params.query, launch, true, false, rq::launch_unset(&params.launch), p, w.stream);
+        st = rq::launch_trace(kind, params.query, launch, true, false, p, w.stream);
     }
     if (st == RQ_OK) st = rq::ao_finish_items_launch(d_bakes, n_bakes, ao_blocks, w.stream);
     for (Piece* pc : batch) {

@@ -58,10 +58,11 @@ typedef enum rq_bvh_kind { RQ_BVH_CWBVH = 0, RQ_BVH_BVH2 = 1 } rq_bvh_kind;
 typedef enum rq_query { RQ_CLOSEST = 0, RQ_ANY = 1 } rq_query;
 
 /* Launch parameters of the persistent trace kernels.  Zero fields take the
- * built-in defaults (or the autotuner's cached choice, see rq_autotune).  With
- * none of the shape, postponing and fetch fields set, a CWBVH launch of a few
- * ten thousand rays or fewer takes a kernel with several lanes per ray
- * instead; step_limit holds for it too. */
+ * built-in defaults (rq_default_launch).  With the default shape, postponing
+ * and fetch values, whether left at zero or named, the library may choose
+ * another kernel: a CWBVH launch of a few ten thousand rays or fewer takes one
+ * with several lanes per ray, a large any-hit batch one with its own stack and
+ * refill sizes.  step_limit holds for all. */
 typedef struct rq_launch {
     int block_size;       /* threads per block: 64, 128, 256 or 512             */
     int blocks_per_sm;    /* persistent grid = SMs x this (0 = occupancy max)   */
@@ -246,7 +247,9 @@ rq_status rq_sharded_trace(rq_sharded_t shards, const rq_ray* rays, rq_hit* hits
 rq_status rq_sharded_destroy(rq_sharded_t shards);
 
 /* Defaults used when rq_launch fields are zero (a negative postpone_ratio
- * turns triangle postponing off). */
+ * turns triangle postponing off); passing them is the same launch as NULL in
+ * rq_trace, rq_trace_ao, the batches, the sharded trace and the server.
+ * rq_trace_instanced has defaults of its own. */
 rq_status rq_default_launch(rq_bvh_kind kind, rq_query query, rq_launch* out);
 
 /* ------------------------------------------------------------ AO ray input */
@@ -371,9 +374,9 @@ rq_status rq_batch_destroy(rq_batch_t batch);
  * Time the candidate launch shapes (block size, shared-memory stack depth,
  * postponing on/off) on the given rays, then, on the fastest shape, the
  * dynamic-fetch refill thresholds (fetch_nd, fetch_nw) and the postponing
- * ratio, and return the fastest.  When cache_path is non-null the choice is
- * stored there keyed by device, BVH kind, query and size class, and later
- * calls read it back.
+ * ratio, and return the fastest.  The default launch is among the candidates.
+ * When cache_path is non-null the choice is stored there keyed by device, BVH
+ * kind, query, size class and kernel revision, and later calls read it back.
  */
 rq_status rq_autotune(rq_ctx_t ctx, rq_scene_t scene, const rq_ray* rays, rq_hit* hits,
                       int64_t count, rq_query query, const char* cache_path, rq_launch* out,
