@@ -196,15 +196,21 @@ constexpr int kMaxItems = 4096;
 constexpr size_t kTableBytes = kMaxItems * (sizeof(rq::TraceItem) + sizeof(rq::AoItem));
 static_assert(sizeof(rq::TraceItem) % 8 == 0 && alignof(rq::AoItem) <= 8, "bake items follow the trace items");
 
-// A bake piece whose surfels and AO lie in pinned memory moves them without
-// copies up to this many surfels: the ray kernel reads the surfels over the
-// link (each by one block, or by every 256 rays of it) and the last kernel
-// writes the AO.  A copy costs the dispatcher ~5 us to queue, and four of them
-// with two kernels and a memset per piece were half of a burst of small
-// requests: 24 of 128 to 32,768 surfels at 32 rays 1,960 -> 1,240 us, 24 of 512
-// 1,070 -> 510 us.  With 65,536 surfels (2.4 MB) at 4 rays the copy engine is
-// as fast or faster (4 requests 650-930 us copied, 720-1,010 us mapped).
-constexpr int64_t kMappedSurfels = 32768;
+// A bake request whose surfels and AO lie in pinned memory moves them without
+// copies when a piece of it has up to this many surfels: the ray kernel reads
+// the surfels over the link (each by one block, or by every 256 rays of it) and
+// the last kernel writes the AO.  A copy costs the dispatcher ~5 us to queue,
+// and four of them with two kernels and a memset per piece were half of a burst
+// of small requests (24 of 512 surfels 1,070 -> 510 us); but copies overlap the
+// other streams' traces, and reads over the link hold up their own.  Bursts of
+// 24 requests, us, mapped / copied (medians of 3-4 processes): 2,000 surfels at
+// 4 rays 464 / 720, 8,000 at 4 780 / 993, 8,000 at 32 2,115 / 2,362; 12,288 at
+// 4 1,284 / 1,154, 16,384 at 32 3,490 / 3,124, 32,768 at 4 2,396 / 1,647.  It
+// holds for the pieces of a large request too: one of 1M surfels at 32 rays in
+// pieces of 8,192 14,300 / 16,100 us.  With many rays to a surfel they are the
+// same from 256 to 1,024 (4 requests of 1,000: 700 / 650, 1,350 / 1,370) and
+// copies 20 % faster at 2,048.
+constexpr int64_t kMappedSurfels = 8192;
 constexpr int kMappedSpp = 256;
 
 }  // namespace
