@@ -1769,7 +1769,11 @@ static ScratchPool& scratch_pool() {
     static ScratchPool* p = new ScratchPool();  // never destroyed: scenes may outlive static objects
     return *p;
 }
-void rq::gpu_built_scene_gone(int device) { scratch_pool().leave(device); }
+void rq::gpu_built_scene_gone(int device, cudaEvent_t scratch_freed) {
+    cudaEventSynchronize(scratch_freed);
+    cudaEventDestroy(scratch_freed);
+    scratch_pool().leave(device);
+}
 
 // One allocation from the pool cut into aligned buffers: laid out first, then
 // made.
@@ -2097,12 +2101,19 @@ static rq_status build_scene(const float* vertices, int64_t nv, const int32_t* i
     float root[20] = {};
     if (st == RQ_OK)
         ok(cudaMemcpyAsync(root, nodes, sizeof(root), cudaMemcpyDeviceToHost, s), "rq_build_scene_gpu");
-    // Freed before the host's last wait: the pool gives back, with the last
-    // scene, only what it has seen the stream let go of.
+    ok(cudaStreamSynchronize(s), "rq_build_scene_gpu");
+    // The pool gives back only what the host has seen the stream let go of, so
+    // the scene keeps an event behind the frees and waits for it when it goes.
+    // (Freeing before the wait above instead has the pool give back all beyond
+    // kPoolKeepBytes in every build and map it again in the next: 2M triangles
+    // 9.9 -> 11.5 ms.)
+    cudaEvent_t freed = nullptr;
+    if (st == RQ_OK) ok(cudaEventCreateWithFlags(&freed, cudaEventDisableTiming), "rq_build_scene_gpu");
     arena.release();
     rm.arena.release();
-    ok(cudaStreamSynchronize(s), "rq_build_scene_gpu");
+    if (st == RQ_OK) ok(cudaEventRecord(freed, s), "rq_build_scene_gpu");
     if (st != RQ_OK) {
+        if (freed) cudaEventDestroy(freed);
         cudaFree(block);
         return st;
     }
@@ -2110,7 +2121,7 @@ static rq_status build_scene(const float* vertices, int64_t nv, const int32_t* i
     sc->kind = RQ_BVH_CWBVH;
     sc->device = device;
     sc->block = block;
-    sc->gpu_built = true;
+    sc->scratch_freed = freed;
     sc->nodes = nodes;
     sc->woop = woop;
     sc->prim_index = prim;

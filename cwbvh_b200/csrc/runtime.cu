@@ -370,7 +370,7 @@ rq_status rq_scene_destroy(rq_scene_t scene) {
         cudaFree((void*)scene->woop);
         if (scene->prim_index) cudaFree((void*)scene->prim_index);
     }
-    if (scene->gpu_built) gpu_built_scene_gone(scene->device);
+    if (scene->scratch_freed) gpu_built_scene_gone(scene->device, scene->scratch_freed);
     delete scene;
     return RQ_OK;
 }

@@ -26,7 +26,7 @@ struct rq_scene {
     int64_t node_f4 = 0, woop_f4 = 0, prim_count = 0;
     bool owned = false;
     void* block = nullptr;   // the one allocation the owned buffers lie in (null: one each)
-    bool gpu_built = false;  // holds its device's build scratch pool
+    cudaEvent_t scratch_freed = nullptr;  // built on the device, holds its build scratch pool: behind the scratch's frees
     float lo[3] = {0.f, 0.f, 0.f};
     float hi[3] = {0.f, 0.f, 0.f};
 };
@@ -46,8 +46,9 @@ void set_last_error(const std::string& msg);
 
 int device_sms(int device);
 
-// A scene that rq_build_scene_gpu made on `device` was destroyed (gpubuild.cu).
-void gpu_built_scene_gone(int device);
+// A scene that rq_build_scene_gpu made on `device` was destroyed (gpubuild.cu);
+// takes its event.
+void gpu_built_scene_gone(int device, cudaEvent_t scratch_freed);
 
 // Fills zero fields of `l` with defaults for this BVH kind / query.
 rq_launch resolve_launch(rq_bvh_kind kind, rq_query q, const rq_launch* l);
