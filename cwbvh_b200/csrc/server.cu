@@ -196,21 +196,27 @@ constexpr int kMaxItems = 4096;
 constexpr size_t kTableBytes = kMaxItems * (sizeof(rq::TraceItem) + sizeof(rq::AoItem));
 static_assert(sizeof(rq::TraceItem) % 8 == 0 && alignof(rq::AoItem) <= 8, "bake items follow the trace items");
 
-// A bake request whose surfels and AO lie in pinned memory moves them without
-// copies when a piece of it has up to this many surfels: the ray kernel reads
-// the surfels over the link (each by one block, or by every 256 rays of it) and
-// the last kernel writes the AO.  A copy costs the dispatcher ~5 us to queue,
-// and four of them with two kernels and a memset per piece were half of a burst
-// of small requests (24 of 512 surfels 1,070 -> 510 us); but copies overlap the
-// other streams' traces, and reads over the link hold up their own.  Bursts of
-// 24 requests, us, mapped / copied (medians of 3-4 processes): 2,000 surfels at
-// 4 rays 464 / 720, 8,000 at 4 780 / 993, 8,000 at 32 2,115 / 2,362; 12,288 at
-// 4 1,284 / 1,154, 16,384 at 32 3,490 / 3,124, 32,768 at 4 2,396 / 1,647.  It
-// holds for the pieces of a large request too: one of 1M surfels at 32 rays in
-// pieces of 8,192 14,300 / 16,100 us.  With many rays to a surfel they are the
-// same from 256 to 1,024 (4 requests of 1,000: 700 / 650, 1,350 / 1,370) and
-// copies 20 % faster at 2,048.
-constexpr int64_t kMappedSurfels = 8192;
+// A bake piece of up to kMappedSurfels surfels whose arrays lie in pinned memory
+// moves them without copies, until the pieces of its launch have read
+// kMappedLaunchSurfels that way: the ray kernel reads the surfels over the link
+// (each by one block, or by every 256 rays of it) and the last kernel writes the
+// AO.  A copy costs the dispatcher ~5 us to queue, and four of them with two
+// kernels and a memset per piece were half of a burst of small requests (24 of
+// 512 surfels 1,070 -> 510 us).  But reads over the link hold up their launch's
+// own rays, where copies overlap the other streams' traces, so the limit that
+// counts is how much a launch reads.  Medians of five processes, us, before
+// requests were read in place / everything copied / no limit to a launch / with
+// the limit: 24 requests of 128 to 32,768 surfels (log-uniform) at 16 rays 1,608
+// / 1,005 / 757 / 708, 12 at 32 892 / 645 / 507 / 469, 24 of 4,096 at 4 1,054 /
+// 718 / 612 / 487, 24 of 16,384 at 16 2,597 / 1,988 / 2,458 / 2,067, 24 of
+// 32,768 at 4 2,260 / 1,654 / 2,199 / 2,164, 8 of them 945 / 654 / 1,031 / 911.
+// (65,536 a launch: the last two 1,976 and 721, but 24 of 128 to 10,000 at 32
+// rays 966 instead of 737; a limit of 8,192 to a request instead: the first
+// 1,290.)  With many rays to a surfel in place and copied are the same from 256
+// to 1,024 (4 requests of 1,000: 700 / 650, 1,350 / 1,370), and copies 20 %
+// faster at 2,048.
+constexpr int64_t kMappedSurfels = 32768;
+constexpr int64_t kMappedLaunchSurfels = 98304;
 constexpr int kMappedSpp = 256;
 
 }  // namespace
@@ -262,6 +268,7 @@ void rq_server::launch_batch(Worker& w, std::vector<Piece*>& batch, int32_t batc
     rq::AoItem* bakes = reinterpret_cast<rq::AoItem*>(w.h_table + bake_at);
     int n_bakes = 0;
     uint32_t ray_blocks = 0, ao_blocks = 0;
+    int64_t in_place = kMappedLaunchSurfels;
     int64_t ray_begin = 0;
     for (size_t k = 0; k < batch.size(); ++k) {
         Piece* pc = batch[k];
@@ -288,7 +295,8 @@ void rq_server::launch_batch(Worker& w, std::vector<Piece*>& batch, int32_t batc
             const float* d_rad = r->host_radius ? reinterpret_cast<float*>(take(4 * n)) : nullptr;
             uint32_t* d_counts = reinterpret_cast<uint32_t*>(take(4 * n));
             rq_ray* d_rays = reinterpret_cast<rq_ray*>(take(n * r->spp * (int64_t)sizeof(rq::Ray)));
-            if (r->map_pos) {
+            if (r->map_pos && n <= in_place) {
+                in_place -= n;
                 d_pos = r->map_pos + 4 * pc->first;
                 d_nrm = r->map_nrm + 4 * pc->first;
                 if (d_rad) d_rad = r->map_radius + pc->first;

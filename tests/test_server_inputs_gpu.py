@@ -13,8 +13,8 @@ def _pinned(x):
     return torch.empty(x.shape, dtype=torch.float32, pin_memory=True).copy_(torch.from_numpy(x)).numpy()
 
 
-# surfels, rays each, rays per launch: whole requests around the most surfels that are read in place, and pieces of
-# 4,000, 1 and 300 surfels with a last one of another size
+# surfels, rays each, rays per launch: whole requests around the most surfels that are read in place (several of them
+# pass what a launch reads in place), and pieces of 4,000, 1 and 300 surfels with a last one of another size
 @pytest.mark.parametrize("n, spp, cap", [(3, 7, 1 << 20), (8191, 2, 1 << 20), (8192, 2, 1 << 20), (8193, 2, 1 << 20),
                                          (32768, 2, 1 << 20), (32769, 2, 1 << 20), (9001, 16, 64000), (5, 33, 33),
                                          (1000, 256, 76800), (70001, 2, 40000)])
