@@ -372,7 +372,8 @@ rq_status rq_autotune_batch(rq_ctx_t ctx, const rq_batch_item* items, int n_item
     // The ring kernels want 4 entries (12 x 800,000 AO rays, 128 threads, 4 / 8
     // / 16: 1,806 / 1,872 / 2,036 us), the others 8 (closest-hit batches 3,537 /
     // 3,504 / 3,515, BVH2 3,289 / 3,216 / 3,219, BVH2 any-hit 2,248 / 2,189 /
-    // 2,188); 16 is nowhere more than 0.3 % ahead of both.
+    // 2,188; 127M closest hits of 64 scenes, 64 threads, 2,252 / 2,335 / 1,949
+    // Mrays/s); 16 is nowhere more than 0.3 % ahead of both.
     const int stacks[] = {4, 8};
     // Sort thresholds: never, items of at least 1M rays, every item.
     const int64_t thresholds[] = {-1, std::min<int64_t>(max_count, 1 << 20), 0};

@@ -1724,7 +1724,9 @@ using namespace rq;
 // up to kPoolKeepBytes between builds while a scene built on the device lives
 // (a new block of memory costs ~330 us to map and ~270 us to unmap, up to
 // several ms now and then; a build of 500,000 triangles takes 4 ms besides).
-// The memory goes back to the device with the last such scene.  A pool is
+// The memory goes back to the device with the last such scene, so a caller that
+// destroys each scene before it builds the next maps it anew every time (500,000
+// triangles 3.6 -> 4.0 ms, and the destruction takes 1.2).  A pool is
 // safe for any number of threads and streams, and hands a block that one
 // stream freed to another only in order.
 constexpr uint64_t kPoolKeepBytes = 256ull << 20;  // the scratch of about a million triangles

@@ -86,7 +86,9 @@ __device__ __forceinline__ void aorays_block(
     const int64_t surfel0 = SMALL ? (int64_t)spp.div((uint32_t)block0) : block0 / spp.d;  // SMALL: n_rays < 2^31
     const uint32_t skip = (uint32_t)(block0 - surfel0 * spp.d);
     const uint32_t here = (uint32_t)(n_rays - block0 < kAoBlock ? n_rays - block0 : kAoBlock);  // rays of the block
-    // skip + here - 1 < spp + 256 <= 2^31: spp fits an int
+    // skip < spp and here <= 256, so the sum is below 2^31 + 255.  From 2^31 on
+    // the division is past FastDiv's general range but still exact: spp is then
+    // above 2^31 - 256, and the quotient 1 far from its ends.
     const uint32_t n_surfels = spp.div(skip + here - 1u) + 1u;
     if (threadIdx.x < n_surfels) {
         const int64_t s = surfel0 + threadIdx.x;

@@ -561,8 +561,10 @@ rq_status rq_device_free(void* p);
  * owns its buffers (rq_scene_destroy).  No reference counterpart (the
  * reference builds on the host with Embree).  Indices outside [0, nv) give
  * RQ_ERR_INVALID_ARG, as do an unknown method and a budget outside
- * [0, 400].  Synchronises `stream` once per tree level (and once per
- * clustering round).
+ * [0, 400].  Vertices are not checked: triangles with infinite or NaN ones are
+ * stored but not found, and may hide others.  Waits for `stream` several times
+ * (every eight tree levels, every six clustering rounds).  Scratch comes from a
+ * memory pool that keeps up to 256 MB while a scene built on the device lives.
  */
 #define RQ_GPU_BUILD_LBVH 0
 #define RQ_GPU_BUILD_PLOC 1
